@@ -644,6 +644,21 @@ void set_relax(SweepArgs &a, int Q, int, double omega) {
     a.rkf[k] = kf[k];
     a.rkl[k] = (float)(rk[k] - (double)kf[k]);
   }
+  // Block fixed point (fixed.cuh), from the exact FP64 omega in extended precision.
+  const long double om = omega, W = Q == 27 ? 1.0L / 27.0L : 1.0L / 9.0L;
+  auto fix = [&](int k, long double x) {
+    const long long v = llrintl(x);
+    a.fx[k].l = (int)(uint32_t)v;
+    a.fx[k].h = (int)((v - a.fx[k].l) >> 32);
+  };
+  a.fx_ok = std::fabs(1.0 - omega) <= 1.0 - 0x1p-20 ? 1 : 0;
+  if (a.fx_ok) {
+    fix(FX_OMC, 0x1p63L * (1.0L - om));
+    fix(FX_T, 0x1p63L * (4.5L * W * om));
+    fix(FX_V, (Q == 27 ? 0x1p60L : 0x1p59L) * (3.0L * W * om));
+    fix(FX_G, 0x1p61L * (W * om));
+    fix(FX_THIRD, 0x1p64L / 3.0L);
+  }
 }
 
 void set_offsets(SweepArgs &a, int Q) {

@@ -6,6 +6,8 @@
 //   D3Q27 "3D MPI+KOKKOS+MPIIO/lbm.cpp:55-218": rest, then +/- pairs (2k-1, 2k).
 #pragma once
 #include <cstdint>
+#include <type_traits>
+#include <utility>
 #include <cuda_fp16.h>
 
 namespace cflbm {
@@ -86,6 +88,34 @@ __host__ __device__ constexpr int mirror(int i, int d) {
     if (L::ex(k) == w0 && L::ey(k) == w1 && L::ez(k) == w2) return k;
   return -1;
 }
+
+// Index of the direction with velocity (ex, ey, ez), -1 if none; and the
+// weight class of direction i (|e_i|^2: 0 rest, 1 axis, 2 face diagonal,
+// 3 corner).
+template <class L>
+__host__ __device__ constexpr int dir_of(int ex, int ey, int ez) {
+  for (int k = 0; k < L::Q; ++k)
+    if (L::ex(k) == ex && L::ey(k) == ey && L::ez(k) == ez) return k;
+  return -1;
+}
+template <class L>
+__host__ __device__ constexpr int wclass(int i) {
+  return L::ex(i) * L::ex(i) + L::ey(i) * L::ey(i) + L::ez(i) * L::ez(i);
+}
+// Pair index k (L::pair(k) = i) of direction i or of its opposite.
+template <class L>
+__host__ __device__ constexpr int pair_of(int i) {
+  for (int k = 0; k < L::NPAIR; ++k)
+    if (L::pair(k) == i || L::opp(L::pair(k)) == i) return k;
+  return -1;
+}
+
+#if defined(__CUDACC__)
+template <class F, int... Is>
+__device__ __forceinline__ void static_for(F &&f, std::integer_sequence<int, Is...>) {
+  (f(std::integral_constant<int, Is>{}), ...);
+}
+#endif
 
 // ---- storage formats ---------------------------------------------------------
 // Store<T>::load/store convert between the stored element and the arithmetic

@@ -55,6 +55,16 @@ __host__ __device__ inline bool mask_solid(const uint32_t *m, int nxw, int ny, i
 constexpr int RK_OMC = 0, RK_W = 1, RK_A = 5, RK_3 = 9, RK_LW = 13, RK_L3 = 14, RK_LA = 15,
               RK_M3 = 16, RK_N = 20;
 
+// Constants of the block fixed-point collision (fixed.cuh): 64-bit integers as
+// balanced limbs h 2^32 + l; with W the lattice's weight constant and u the
+// velocity scale Fx::U,
+//   FX_OMC 2^63 (1 - omega), FX_T 2^63 4.5 W omega, FX_V 2^(63-U) 3 W omega,
+//   FX_G 2^61 W omega, FX_THIRD 2^64 / 3.
+enum { FX_OMC = 0, FX_T, FX_V, FX_G, FX_THIRD, FX_N };
+struct FxConst {
+  int h, l;
+};
+
 struct SweepArgs {
   Layout L;
   const void *fa;        // post-collision state of this step (ghosts filled)
@@ -69,6 +79,8 @@ struct SweepArgs {
   double rk[RK_N];
   float rkf[RK_N];
   float rkl[RK_N];
+  FxConst fx[FX_N];      // block fixed-point constants (FP64 arithmetic)
+  int fx_ok;             // 1: the rate is within their range
   bool f16_sr;           // FP16 storage: stochastic rounding of stores (else nearest)
   // Per direction I, in elements: doff = I * S (the population's storage
   // offset) and poff = doff - L.off(e_I) (the plain pull's source), kernel

@@ -34,14 +34,10 @@
 #pragma once
 #include <type_traits>
 #include <utility>
+#include "fixed.cuh"
 #include "solver.cuh"
 
 namespace cflbm {
-
-template <class F, int... Is>
-__device__ __forceinline__ void static_for(F &&f, std::integer_sequence<int, Is...>) {
-  (f(std::integral_constant<int, Is>{}), ...);
-}
 
 // Collision arithmetic over V = float, double, float2 (two cells per thread,
 // GB300's packed FFMA2/FADD2/FMUL2) or df64 (double-float, below).  Every operation is explicitly rounded, so
@@ -142,27 +138,6 @@ template <> struct VA<df64> {
   __device__ static df64 fma(df64 a, df64 b, df64 c) { return add(mul(a, b), c); }
 };
 
-
-// Index of the direction with velocity (ex, ey, ez), -1 if none; and the
-// weight class of direction i (|e_i|^2: 0 rest, 1 axis, 2 face diagonal,
-// 3 corner).
-template <class L>
-__host__ __device__ constexpr int dir_of(int ex, int ey, int ez) {
-  for (int k = 0; k < L::Q; ++k)
-    if (L::ex(k) == ex && L::ey(k) == ey && L::ez(k) == ez) return k;
-  return -1;
-}
-template <class L>
-__host__ __device__ constexpr int wclass(int i) {
-  return L::ex(i) * L::ex(i) + L::ey(i) * L::ey(i) + L::ez(i) * L::ez(i);
-}
-// Pair index k (L::pair(k) = i) of direction i or of its opposite.
-template <class L>
-__host__ __device__ constexpr int pair_of(int i) {
-  for (int k = 0; k < L::NPAIR; ++k)
-    if (L::pair(k) == i || L::opp(L::pair(k)) == i) return k;
-  return -1;
-}
 
 // Relaxation constants of a sweep (SweepArgs::rk, host-computed per handle):
 //   rk[0]      = 1 - omega
@@ -424,10 +399,17 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_kernel(const 
     f[i] = SF::template load<A, L>(fa + i * S + c - a.L.off(L::ex(i), L::ey(i), L::ez(i)),
                                    a.L.fbase[i]);
 
+  const long long cell = ((long long)z * a.L.ny + y) * a.L.nx + x;
+  const bool solid = mask_solid(a.mask, a.nxw, a.L.ny, x, y, z);
+  if constexpr (std::is_same<A, double>::value) {
+    const bool in = a.ref_override && x == 0;
+    if (fixed_cell<L, SF>(f, solid, in, in ? a.inlet_u[(long long)z * a.L.ny + y] : 0.0,
+                          a.ref_override && x == a.L.nx - 1, cell, true, fb, c, S, a))
+      return;
+  }
   A rho3, ux, uy, uz;
   moments<L, A, SF>(f, rho3, ux, uy, uz);
-  const long long cell = ((long long)z * a.L.ny + y) * a.L.nx + x;
-  if (mask_solid(a.mask, a.nxw, a.L.ny, x, y, z)) {
+  if (solid) {
     rho3 = A(0); ux = A(0); uy = A(0); uz = A(0);
   }
   if (a.ref_override) {
@@ -925,12 +907,15 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_channel_kerne
         },
         std::make_integer_sequence<int, Q>{});
   }
+  const long long cell = ((long long)z * ny + y) * nx + x;
+  if constexpr (std::is_same<A, double>::value) {
+    if (fixed_cell<L, SF>(f, solid_here, false, 0.0, false, cell, valid, fb, c, S, a)) return;
+  }
   A rho3, ux, uy, uz;
   moments<L, A, SF>(f, rho3, ux, uy, uz);
   if (solid_here) {
     rho3 = A(0); ux = A(0); uy = A(0); uz = A(0);
   }
-  const long long cell = ((long long)z * ny + y) * nx + x;
   finish_cell<L, SF, A, E>(f, rho3, ux, uy, uz, cell, valid, fb, c, S, a);
 }
 
