@@ -642,7 +642,6 @@ void set_relax(SweepArgs &a, int Q, int, double omega) {
   for (int k = 0; k < RK_N; ++k) {
     a.rk[k] = rk[k];
     a.rkf[k] = kf[k];
-    a.rkl[k] = (float)(rk[k] - (double)kf[k]);
   }
   // Block fixed point (fixed.cuh), from the exact FP64 omega in extended precision.
   const long double om = omega, W = Q == 27 ? 1.0L / 27.0L : 1.0L / 9.0L;
@@ -697,7 +696,6 @@ SweepArgs channel_args(const cflbm_handle *h, const void *fa, void *fb, bool wri
   for (int i = 0; i < h->Q; ++i) {
     sa.f_in[i] = h->f_in[i];
     sa.f_in_f[i] = (float)h->f_in[i];
-    sa.f_in_l[i] = (float)(h->f_in[i] - (double)sa.f_in_f[i]);
   }
   // Grid of the force launch beside the sweep: one boundary cell per thread,
   // at most one block per SM.

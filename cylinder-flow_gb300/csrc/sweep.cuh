@@ -40,7 +40,7 @@
 namespace cflbm {
 
 // Collision arithmetic over V = float, double, float2 (two cells per thread,
-// GB300's packed FFMA2/FADD2/FMUL2) or df64 (double-float, below).  Every operation is explicitly rounded, so
+// GB300's packed FFMA2/FADD2/FMUL2).  Every operation is explicitly rounded, so
 // the compiler neither contracts nor reorders: a cell gets the same bits from
 // every kernel that collides it, scalar or packed.
 template <class V> struct VA;
@@ -72,87 +72,19 @@ template <> struct VA<float2> {
   __device__ static float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 };
 
-// Double-float arithmetic (df64, lattice.cuh)
-// from published error-free transformations: Knuth's TwoSum, Dekker's Fast2Sum
-// and the FMA-based exact product (Dekker, "A floating-point technique for
-// extending the available precision", Numer. Math. 18, 1971; Joldes, Muller and
-// Popescu, "Tight and rigorous error bounds for basic building blocks of
-// double-word arithmetic", ACM TOMS 44(2), 2017).
-//   add: Dekker's double-word sum (their Algorithm 5, "sloppy"): TwoSum of the
-//        high parts, the low parts added to its error, Fast2Sum -- 11
-//        operations; error <= 2u^2 (|x| + |y|) (u = 2^-24), relative to the
-//        operands, not the result, which is what a collision needs: every
-//        population is compared to the field, not to itself;
-//   mul: the exact product of the high parts plus the cross terms (the
-//        lo*lo term, ~u^2 of the product, dropped), Fast2Sum -- 8 operations;
-//        relative error <= 4u^2.
-// T = float (the df64 arithmetic of one cell per thread).
-template <class T> struct DWops {
-  using O = VA<T>;
-  __device__ static T neg(T a) { return O::sub(O::splat(0.0f), a); }
-  __device__ static void two_sum(T a, T b, T &s, T &t) {
-    s = O::add(a, b);
-    const T ap = O::sub(s, b), bp = O::sub(s, ap);
-    t = O::add(O::sub(a, ap), O::sub(b, bp));
-  }
-  __device__ static void fast_two_sum(T a, T b, T &s, T &t) {
-    s = O::add(a, b);
-    t = O::sub(b, O::sub(s, a));
-  }
-  __device__ static void add(T xh, T xl, T yh, T yl, T &zh, T &zl) {
-    T sh, e;
-    two_sum(xh, yh, sh, e);
-    e = O::add(e, O::add(xl, yl));
-    fast_two_sum(sh, e, zh, zl);
-  }
-  __device__ static void mul(T xh, T xl, T yh, T yl, T &zh, T &zl) {
-    const T ch = O::mul(xh, yh);
-    const T cl1 = O::fma(xh, yh, neg(ch));
-    const T cl2 = O::fma(xl, yh, O::mul(xh, yl));
-    fast_two_sum(ch, O::add(cl1, cl2), zh, zl);
-  }
-};
-template <> __device__ __forceinline__ float DWops<float>::neg(float a) { return -a; }
-template <> __device__ __forceinline__ float2 DWops<float2>::neg(float2 a) {
-  return make_float2(-a.x, -a.y);
-}
-
-template <> struct VA<df64> {
-  using S = double;
-  using D = DWops<float>;
-  __device__ static df64 splat(double s) {  // constants: folded at compile time
-    const float h = (float)s;
-    return df64(h, (float)(s - (double)h));
-  }
-  __device__ static df64 add(df64 x, df64 y) {
-    df64 z;
-    D::add(x.hi, x.lo, y.hi, y.lo, z.hi, z.lo);
-    return z;
-  }
-  __device__ static df64 sub(df64 x, df64 y) { return add(x, df64(-y.hi, -y.lo)); }
-  __device__ static df64 mul(df64 x, df64 y) {
-    df64 z;
-    D::mul(x.hi, x.lo, y.hi, y.lo, z.hi, z.lo);
-    return z;
-  }
-  __device__ static df64 fma(df64 a, df64 b, df64 c) { return add(mul(a, b), c); }
-};
-
-
 // Relaxation constants of a sweep (SweepArgs::rk, host-computed per handle):
 //   rk[0]      = 1 - omega
 //   rk[1 + c]  = omega w_c         (Kw, weight class c)
 //   rk[5 + c]  = 4.5 omega w_c     (Ka)
 //   rk[9 + c]  = 3 omega w_c       (K3)
 //   rk[16 + c] = -6 omega w_c      (-2 K3)
-// in FP64 (rk) and as the FP32 remainder rk - rkf (rkl), which with rkf forms
-// the double-float constant.
+// in FP64 (rk).
 // The FP32 set (rkf) is not rk rounded one by one: with Om = 1 - rkf[0] (exact)
 // its values satisfy, as real numbers, the identities behind mass and momentum
 // conservation of the collision,
 //   sum_i Kw_i = Om,   sum_i K3_i e_ix^2 = Om,   sum_i Ka_i e_ix^2 = 1.5 Om,
 // the rest class's Kw and the face class's K3 and Ka taking the remainder as a
-// double-float pair (rkf[RK_W], rkf[RK_LW]), (rkf[RK_3 + 1], rkf[RK_L3]),
+// pair hi + lo (rkf[RK_W], rkf[RK_LW]), (rkf[RK_3 + 1], rkf[RK_L3]),
 // (rkf[RK_A + 1], rkf[RK_LA]).  Constants rounded one by one miss these by a
 // few 1e-8 per step -- a standing mass and momentum source that moves the
 // period-averaged drag of the 400x100 channel by ~1e-3.
@@ -166,9 +98,6 @@ template <> __device__ __forceinline__ float rconst<float>(const SweepArgs &a, i
 }
 template <> __device__ __forceinline__ float2 rconst<float2>(const SweepArgs &a, int k) {
   return make_float2(a.rkf[k], a.rkf[k]);
-}
-template <> __device__ __forceinline__ df64 rconst<df64>(const SweepArgs &a, int k) {
-  return df64(a.rkf[k], a.rkl[k]);
 }
 
 
@@ -245,9 +174,7 @@ __device__ __forceinline__ void bgk_relax_each(G &&get, Pt &&put, V rho3, V ux, 
           sm = O::sub(sym, asym);
         } else {
           // FP64: Horner in e.u, then the odd part's sign flip, 3 operations
-          // for both (5 per pair instead of 7, 26 fewer per D3Q27 cell; a
-          // double-float FMA costs more than the product and sum it replaces:
-          // 7,683 against 7,764 M cell updates/s on 512x128x128, not used there)
+          // for both (5 per pair instead of 7, 26 fewer per D3Q27 cell)
           sp = O::fma(eu, O::fma(rconst<V>(a, RK_A + c), eu, rconst<V>(a, RK_3 + c)), Ac[c]);
           sm = O::fma(rconst<V>(a, RK_M3 + c), eu, sp);
         }
@@ -444,11 +371,10 @@ template <int Q, int I> struct DirC {
 
 
 // Inlet equilibrium population in the arithmetic type (no FP64 conversion in
-// FP32 sweeps; f_in_f + f_in_l for double-float).
+// FP32 sweeps).
 template <class A>
 __device__ __forceinline__ A inlet_pop(const SweepArgs &a, int i) {
-  if constexpr (std::is_same<A, df64>::value) return df64(a.f_in_f[i], a.f_in_l[i]);
-  else if constexpr (sizeof(A) == 8) return a.f_in[i];
+  if constexpr (sizeof(A) == 8) return a.f_in[i];
   else return a.f_in_f[i];
 }
 
@@ -677,10 +603,7 @@ __device__ __forceinline__ void channel_listed_cell(const SweepArgs &a, int x, i
 // owns cells x and x + 32, whose loads and stores share their address (the
 // second is an immediate 32 elements further).  Moments and BGK run once on
 // the pair type P = float2 with GB300's packed FFMA2/FADD2/FMUL2, halving the
-// arithmetic instructions of the issue-bound FP32-collision forms.  (A
-// double-float pair type needs ~250 registers for two cells' 27 populations;
-// at 2-3 blocks per SM it ran at 2.9-3.9 G cell updates/s against 7.5 for one
-// cell per thread at 5 blocks per SM, D3Q27 512x128x128.)  A pair holding a listed
+// arithmetic instructions of the issue-bound FP32-collision forms.  A pair holding a listed
 // tile pulls through pull_pair_listed (face-state tables and link words), or,
 // with LISTED1 in the kernel, takes its two cells one after the other through
 // channel_listed_cell (the same values: lane for lane the packed operations

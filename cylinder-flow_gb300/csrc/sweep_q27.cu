@@ -4,11 +4,7 @@
 namespace cflbm {
 
 cudaError_t launch_sweep_q27(int store, int compute, const SweepArgs &a, cudaStream_t s) {
-  // Double-float sweep: 5 blocks per SM (96 registers; measured at 512x128x128:
-  // 3 / 4 / 5 per SM give 3,961 / 3,955 / 4,154 M cell updates/s).
-  if (compute == COMPUTE_DF64)
-    return store == STORE_F64 ? launch_sweep_t<27, double, df64, 5>(a, s) : cudaErrorInvalidValue;
-  if (compute == COMPUTE_F64) {
+  if (compute != COMPUTE_F32) {
     // Block fixed point (fixed.cuh): 5 blocks per SM (96 registers).  REF3D
     // 257x97x97, 20 steps and the fields: 5.51 / 5.46 ms at 5 / 6 per SM (6 spills
     // 130 bytes); FP64 operations at 3 per SM: 15.17 ms.
@@ -29,12 +25,7 @@ cudaError_t launch_sweep_q27(int store, int compute, const SweepArgs &a, cudaStr
 
 cudaError_t launch_sweep_channel_q27(int store, int compute, const SweepArgs &a,
                                       cudaStream_t s, const SweepFork *fk) {
-  // Double-float channel sweep: 5 blocks per SM (102 registers; 3 / 4 / 5 / 6
-  // per SM give 6,839 / 6,972 / 7,468 / 7,434 M cell updates/s at 512x128x128).
-  if (compute == COMPUTE_DF64)
-    return store == STORE_F64 ? launch_sweep_channel_t<27, double, df64, 5, 2>(a, s, fk)
-                              : cudaErrorInvalidValue;
-  if (compute == COMPUTE_F64) {
+  if (compute != COMPUTE_F32) {
     // Block fixed point: 512x128x128, 10 steps and the fields: 9.67 / 8.39 / 8.55 ms
     // at 4 / 5 / 6 per SM; FP64 operations at 3 per SM: 22.78 ms.
     switch (store) {
@@ -54,10 +45,7 @@ cudaError_t launch_sweep_channel_q27(int store, int compute, const SweepArgs &a,
 
 cudaError_t launch_macros_channel_q27(int store, int compute, const SweepArgs &a,
                                       cudaStream_t s) {
-  if (compute == COMPUTE_DF64)
-    return store == STORE_F64 ? launch_macros_channel_t<27, double, df64>(a, s)
-                              : cudaErrorInvalidValue;
-  if (compute == COMPUTE_F64) {
+  if (compute != COMPUTE_F32) {
     switch (store) {
       case STORE_F64: return launch_macros_channel_t<27, double, double>(a, s);
       case STORE_F32: return launch_macros_channel_t<27, float, double>(a, s);

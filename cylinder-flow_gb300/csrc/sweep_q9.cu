@@ -4,9 +4,7 @@
 namespace cflbm {
 
 cudaError_t launch_sweep_q9(int store, int compute, const SweepArgs &a, cudaStream_t s) {
-  if (compute == COMPUTE_DF64)
-    return store == STORE_F64 ? launch_sweep_t<9, double, df64, 4>(a, s) : cudaErrorInvalidValue;
-  if (compute == COMPUTE_F64) {
+  if (compute != COMPUTE_F32) {
     switch (store) {
       case STORE_F64: return launch_sweep_t<9, double, double, 4>(a, s);
       case STORE_F32: return launch_sweep_t<9, float, double, 4>(a, s);
@@ -24,10 +22,7 @@ cudaError_t launch_sweep_q9(int store, int compute, const SweepArgs &a, cudaStre
 
 cudaError_t launch_sweep_channel_q9(int store, int compute, const SweepArgs &a,
                                      cudaStream_t s, const SweepFork *fk) {
-  if (compute == COMPUTE_DF64)
-    return store == STORE_F64 ? launch_sweep_channel_t<9, double, df64, 4, 2>(a, s, fk)
-                              : cudaErrorInvalidValue;
-  if (compute == COMPUTE_F64) {
+  if (compute != COMPUTE_F32) {
     switch (store) {
       case STORE_F64: return launch_sweep_channel_t<9, double, double, 4, 2>(a, s, fk);
       case STORE_F32: return launch_sweep_channel_t<9, float, double, 4, 2>(a, s, fk);
@@ -45,10 +40,7 @@ cudaError_t launch_sweep_channel_q9(int store, int compute, const SweepArgs &a,
 
 cudaError_t launch_macros_channel_q9(int store, int compute, const SweepArgs &a,
                                       cudaStream_t s) {
-  if (compute == COMPUTE_DF64)
-    return store == STORE_F64 ? launch_macros_channel_t<9, double, df64>(a, s)
-                              : cudaErrorInvalidValue;
-  if (compute == COMPUTE_F64) {
+  if (compute != COMPUTE_F32) {
     switch (store) {
       case STORE_F64: return launch_macros_channel_t<9, double, double>(a, s);
       case STORE_F32: return launch_macros_channel_t<9, float, double>(a, s);
