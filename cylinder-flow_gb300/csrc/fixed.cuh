@@ -119,22 +119,11 @@ __device__ __forceinline__ double fx_to_double(long long x, int s20) {
   return __longlong_as_double(u == 0 ? 0 : (long long)(r | ((unsigned long long)sg << 63)));
 }
 
-// Collision and store of one cell with FP64 arithmetic.  f: the pulled
-// populations.  solid: p = u = 0; inlet: u = (ux_in, 0, 0); outlet: p = 0 (the
-// reference profiles' rules).  Returns false, with nothing written, where the
-// format does not cover the cell.
-template <class L, class SF, class E>
-__device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inlet, double ux_in,
-                                           bool outlet, long long cell, bool store,
-                                           E *__restrict__ fb, long long c, long long S,
-                                           const SweepArgs &a) {
-  constexpr int D = L::D;
-  const int eb = fx_exponent<L>(f, inlet && !solid ? ux_in : 0.0);
-  double s = 1.0;
-  if (a.alpha) s = __dsub_rn(1.0, (double)a.alpha[cell]);
-  if (!a.fx_ok || eb > FX_EMAX || !(fabs(s) <= 1.0)) return false;
-
-  long long q[L::Q];
+// The populations as integers q_i and their moments: the cascade of moments_get
+// with the weights' factor 4 between a line's middle and its ends.
+template <class L>
+__device__ __forceinline__ void fx_moments(const double *f, int eb, long long *q, long long &mr,
+                                           long long *mu) {
   const int in20 = (FX_P + 1023 - eb) << 20;
   static_for(
       [&](auto ic) {
@@ -142,11 +131,7 @@ __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inl
         q[I] = __double2ll_rn(scale_bits(f[I], in20 - Fx<L>::k(wclass<L>(I)) * (1 << 20)));
       },
       std::make_integer_sequence<int, L::Q>{});
-
-  // Moments: the cascade of moments_get with the weights' factor 4 between a
-  // line's middle and its ends.
-  long long mr, mu[3] = {0, 0, 0};
-  if constexpr (D == 3) {
+  if constexpr (L::D == 3) {
     long long s0[3][3], s1[3][3];
     static_for(
         [&](auto kc) {
@@ -180,7 +165,39 @@ __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inl
     mr = s0[0] + s0[2] + 4 * s0[1];
     mu[0] = 4 * (s0[2] - s0[0]);
     mu[1] = 4 * (s1[0] + s1[2] + 4 * s1[1]);
+    mu[2] = 0;
   }
+}
+
+// u, v, w and p = rho3 / 3 of one cell in FP64 (null pointers: not wanted).
+template <class L>
+__device__ __forceinline__ void fx_store_macros(const SweepArgs &a, long long cell, int eb,
+                                                long long mr, const long long *mu) {
+  const double su = __hiloint2double((eb - FX_P - Fx<L>::U) << 20, 0);
+  const double sr = __hiloint2double((eb - FX_P - Fx<L>::R) << 20, 0);
+  if (a.mu) a.mu[cell] = __dmul_rn(__ll2double_rn(mu[0]), su);
+  if (a.mv) a.mv[cell] = __dmul_rn(__ll2double_rn(mu[1]), su);
+  if (a.mw) a.mw[cell] = __dmul_rn(__ll2double_rn(mu[2]), su);
+  if (a.mp) a.mp[cell] = __ddiv_rn(__dmul_rn(__ll2double_rn(mr), sr), 3.0);
+}
+
+// Collision and store of one cell with FP64 arithmetic.  f: the pulled
+// populations.  solid: p = u = 0; inlet: u = (ux_in, 0, 0); outlet: p = 0 (the
+// reference profiles' rules).  Returns false, with nothing written, where the
+// format does not cover the cell.
+template <class L, class SF, class E>
+__device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inlet, double ux_in,
+                                           bool outlet, long long cell, bool store,
+                                           E *__restrict__ fb, long long c, long long S,
+                                           const SweepArgs &a) {
+  constexpr int D = L::D;
+  const int eb = fx_exponent<L>(f, inlet && !solid ? ux_in : 0.0);
+  double s = 1.0;
+  if (a.alpha) s = __dsub_rn(1.0, (double)a.alpha[cell]);
+  if (!a.fx_ok || eb > FX_EMAX || !(fabs(s) <= 1.0)) return false;
+
+  long long q[L::Q], mr, mu[3];
+  fx_moments<L>(f, eb, q, mr, mu);
   if (solid) mr = mu[0] = mu[1] = mu[2] = 0;
   if (inlet) {
     mu[0] = __double2ll_rn(scale_bits(ux_in, (FX_P + Fx<L>::U + 1023 - eb) << 20));
@@ -188,14 +205,7 @@ __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inl
   }
   if (outlet) mr = 0;
 
-  if (a.mu && store) {
-    const double su = __hiloint2double((eb - FX_P - Fx<L>::U) << 20, 0);
-    const double sr = __hiloint2double((eb - FX_P - Fx<L>::R) << 20, 0);
-    a.mu[cell] = __dmul_rn(__ll2double_rn(mu[0]), su);
-    a.mv[cell] = __dmul_rn(__ll2double_rn(mu[1]), su);
-    a.mw[cell] = __dmul_rn(__ll2double_rn(mu[2]), su);
-    a.mp[cell] = __ddiv_rn(__dmul_rn(__ll2double_rn(mr), sr), 3.0);
-  }
+  if (a.mu && store) fx_store_macros<L>(a, cell, eb, mr, mu);
   if (a.alpha) {  // u (1 - alpha): the factor at 2^62, the product back by 4
     const Limbs sl = limbs(__double2ll_rn(__dmul_rn(s, 4611686018427387904.0)));
 #pragma unroll

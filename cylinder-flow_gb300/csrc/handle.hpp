@@ -32,7 +32,9 @@ struct cflbm_handle {
   unsigned *d_face_bb = nullptr;         // no-slip face bounce-back bits per face state
   // Channel profile: the steps do not write u, v, w, p; the fields of the last
   // step are formed on request from the state it read (fB after the step).
-  bool macros_pending = false;
+  // Once handed straight to a caller's device arrays (macros_direct) they stay
+  // pending: a second request forms them in d_mu .. d_mp.
+  bool macros_pending = false, macros_direct = false;
   int n_slow = 0;
   double f_in[27] = {0};        // inlet equilibrium (channel profile)
   int4 *d_links = nullptr;
