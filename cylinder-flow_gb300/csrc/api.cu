@@ -75,10 +75,6 @@ void free_handle(cflbm_handle *h) {
   for (cudaGraphExec_t g : h->graph_exec)
     if (g) cudaGraphExecDestroy(g);
   if (h->ev_sync) cudaEventDestroy(h->ev_sync);
-  if (h->fork.side) cudaStreamSynchronize(h->fork.side);
-  if (h->fork.fork) cudaEventDestroy(h->fork.fork);
-  if (h->fork.join) cudaEventDestroy(h->fork.join);
-  if (h->fork.side) cudaStreamDestroy(h->fork.side);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
 }
@@ -291,16 +287,6 @@ int cflbm_create(const cflbm_config *cfg, cflbm_handle **out) {
   CK_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
   CK_CUDA(cudaEventCreateWithFlags(&h->ev_sync, cudaEventDisableTiming));
   CK_CUDA(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, cfg->device));
-  if (cfg->profile == CFLBM_PROFILE_CHANNEL) {
-    // Side stream of the channel step's force kernel, at the highest priority
-    // so its blocks are scheduled ahead of the sweep's.
-    int lo = 0, hi = 0;
-    CK_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-    CK_CUDA(cudaStreamCreateWithPriority(&h->fork.side, cudaStreamNonBlocking, hi));
-    CK_CUDA(cudaEventCreateWithFlags(&h->fork.fork, cudaEventDisableTiming));
-    CK_CUDA(cudaEventCreateWithFlags(&h->fork.join, cudaEventDisableTiming));
-  }
-
   // Layout: ghosts as the profile needs them (the reference's 2 or 3 layers,
   // 1 for the channel), rows padded to 128 bytes with >= 4 spare elements past
   // the last ghost (the reference's wall pass reads two cells beyond the ring).
@@ -447,7 +433,7 @@ int cflbm_create(const cflbm_config *cfg, cflbm_handle **out) {
     if ((rc = dev_alloc_t(h, &h->d_links_bits, 32 * (size_t)total + 32))) return rc;
     CK_CUDA(launch_setup_list(sa, h->d_tile_slow, chunk, h->d_mask, bits, h->d_tile_index,
                               h->d_slow_tiles, h->d_links_bits, h->stream));
-    // The force launch's cells: the fluid cells with solid links, one thread
+    // The force's cells: the fluid cells with solid links, one thread
     // each.  One warp per listed tile with such cells (about 9,000 of the
     // 17,000 listed tiles of the D3Q27 512x128x128 cylinder) left most lanes
     // idle and held its registers for 53 us per step beside the FP16 sweep.
@@ -698,8 +684,7 @@ SweepArgs channel_args(const cflbm_handle *h, const void *fa, void *fb, bool wri
     sa.f_in[i] = h->f_in[i];
     sa.f_in_f[i] = (float)h->f_in[i];
   }
-  // Grid of the force launch beside the sweep: one boundary cell per thread,
-  // at most one block per SM.
+  // Blocks of the force: one boundary cell per thread, at most one block per SM.
   const long long fthreads = SWEEP_BX * SWEEP_BY;
   sa.bnd_blocks = (int)std::max<long long>(
       1, std::min<long long>((h->n_bcells + fthreads - 1) / fthreads, (long long)h->sms));
@@ -749,7 +734,7 @@ static int one_step(cflbm_handle *h, bool write_macros) {
     (void)write_macros;
     const SweepArgs sa = channel_args(h, h->fA, h->fB, false);
     if (h->timing && (trc = record_event(h, &ts0))) return trc;
-    CK_CUDA(launch_sweep_channel(Q, st, h->cfg.compute, sa, h->stream, &h->fork));
+    CK_CUDA(launch_sweep_channel(Q, st, h->cfg.compute, sa, h->stream));
     if (h->timing) {
       if ((trc = record_event(h, &ts1))) return trc;
       h->sweep_ev.push_back({ts0, ts1});
@@ -845,7 +830,7 @@ int cflbm_step(cflbm_handle *h, int nsteps) {
         return rc;
       }
       CK_CUDA(ec);
-      cudaError_t ei = cudaGraphInstantiate(&h->graph_exec[par], g, cudaGraphInstantiateFlagUseNodePriority);
+      cudaError_t ei = cudaGraphInstantiate(&h->graph_exec[par], g, 0);
       cudaGraphDestroy(g);
       CK_CUDA(ei);
       h->launches_per_step = (launches() - n0) / GRAPH_STEPS;

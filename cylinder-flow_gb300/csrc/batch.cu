@@ -52,7 +52,11 @@ struct cflbm_batch {
   long long cells = 0;
   double bytes_per_cell = 0;
   cudaEvent_t done = nullptr;
-  cflbm::SweepFork fork{nullptr, nullptr, nullptr};  // solid-work kernel beside the fast one
+  // The solid-work kernel runs beside the fast one: side stream, fork and join.
+  struct {
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+  } fork;
   std::vector<double> tune_ms;  // timing of each candidate (for cflbm_batch_info)
 };
 

@@ -479,10 +479,8 @@ cudaError_t launch_sweep(int Q, int store, int compute, const SweepArgs &a, cuda
   return Q == 9 ? launch_sweep_q9(store, compute, a, s) : launch_sweep_q27(store, compute, a, s);
 }
 
-cudaError_t launch_sweep_channel_q9(int store, int compute, const SweepArgs &a, cudaStream_t s,
-                                     const SweepFork *fk);
-cudaError_t launch_sweep_channel_q27(int store, int compute, const SweepArgs &a, cudaStream_t s,
-                                      const SweepFork *fk);
+cudaError_t launch_sweep_channel_q9(int store, int compute, const SweepArgs &a, cudaStream_t s);
+cudaError_t launch_sweep_channel_q27(int store, int compute, const SweepArgs &a, cudaStream_t s);
 
 cudaError_t launch_macros_channel_q9(int store, int compute, const SweepArgs &a, cudaStream_t s);
 cudaError_t launch_macros_channel_q27(int store, int compute, const SweepArgs &a,
@@ -505,9 +503,9 @@ cudaError_t launch_stream_state(int Q, int store, const SweepArgs &a, bool ref, 
 }
 
 cudaError_t launch_sweep_channel(int Q, int store, int compute, const SweepArgs &a,
-                                 cudaStream_t s, const SweepFork *fk) {
-  return Q == 9 ? launch_sweep_channel_q9(store, compute, a, s, fk)
-                : launch_sweep_channel_q27(store, compute, a, s, fk);
+                                 cudaStream_t s) {
+  return Q == 9 ? launch_sweep_channel_q9(store, compute, a, s)
+                : launch_sweep_channel_q27(store, compute, a, s);
 }
 
 // Dispatch helper: run F<Q, ST> for the runtime (Q, store).

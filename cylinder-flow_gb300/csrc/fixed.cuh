@@ -42,7 +42,7 @@ constexpr int FX_EMIN = 1023 - 900;  // smaller ones are raised to it
 // operations: 22.78); REF3D 257x97x97, 20 steps: 6.43 / 6.02 / 5.80 / 5.65 / 5.51
 // / 5.43 / 5.58 (15.17); D2Q9 400x100, 400 steps: 2.78 ms for none, 2.70 for all 9
 // (3.11).
-constexpr int FX_NINT = 18;
+template <class L> constexpr int fx_nint = L::D == 3 ? 18 : 4;
 
 // Shift of the weight of class c = |e|^2 (w = W 2^k), the scale of the velocity
 // sums (u = M 2^(E - FX_P - FX_U)) and of rho3 (FX_R).
@@ -241,7 +241,7 @@ __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inl
     constexpr int I = decltype(ic)::value;
     const long long x = mul_hi(q[I], a.fx[FX_OMC], eq);
     double r;
-    if constexpr (I < FX_NINT) {
+    if constexpr (I < fx_nint<L>) {
       r = fx_to_double(x, out20 + (1023 + Fx<L>::k(wclass<L>(I))) * (1 << 20));
     } else {
       const double d = __ll2double_rn(x);

@@ -156,7 +156,9 @@ __device__ __forceinline__ float d2f_bits(double d) {
   return __uint_as_float(t | (hi & 0x80000000u));
 }
 
-// Storage codecs: load/store (global memory) and decode (an element already
+// Storage codecs: load/store (global memory; ordinary cached loads, not the
+// read-only path: a kernel launched while its predecessor still writes the state
+// reads it after griddepcontrol.wait) and decode (an element already
 // read, e.g. from shared memory) convert between the stored element and the
 // arithmetic type A, so the arithmetic always sees the population itself.
 // `base` is the storage offset of the population (Layout::fbase): 0 for FP64 and
@@ -172,8 +174,8 @@ template <> struct Store<double> {
   }
   template <class A, class L>
   __device__ static A load(const elem *p, float) {
-    if constexpr (sizeof(A) == 4) return d2f_bits(__ldg(p));
-    else return static_cast<A>(__ldg(p));
+    if constexpr (sizeof(A) == 4) return d2f_bits(__ldca(p));
+    else return static_cast<A>(__ldca(p));
   }
   template <class A, class L>
   __device__ static void store(elem *p, A v, float, unsigned, bool) {
@@ -187,7 +189,7 @@ template <> struct Store<float> {
   template <class A>
   __device__ static A decode(elem v, float) { return static_cast<A>(v); }
   template <class A, class L>
-  __device__ static A load(const elem *p, float) { return static_cast<A>(__ldg(p)); }
+  __device__ static A load(const elem *p, float) { return static_cast<A>(__ldca(p)); }
   template <class A, class L>
   __device__ static void store(elem *p, A v, float, unsigned, bool) { *p = static_cast<float>(v); }
 };
@@ -249,7 +251,7 @@ template <> struct Store<F16Dev> {
     else return __fma_rn((double)h, 1.0 / F16_SCALE, (double)base);
   }
   template <class A, class L>
-  __device__ static A load(const elem *p, float base) { return decode<A>(__ldg(p), base); }
+  __device__ static A load(const elem *p, float base) { return decode<A>(__ldca(p), base); }
   template <class A, class L>
   __device__ static void store(elem *p, A v, float base, unsigned key, bool sr) {
     float sv;

@@ -111,7 +111,8 @@ struct SweepArgs {
   double *hist;          // force history, 3 doubles per step
   long long *step;       // device step counter (history slot = step % cap)
   long long cap;
-  int bnd_blocks;        // grid of the force launch (at most one block per SM)
+  int bnd_blocks;        // blocks of the force (at most one per SM; 0: not formed)
+  int force_span;        // leading grid rows (2-D) or planes (3-D) of the sweep that form it
   int sms;               // multiprocessors of the device
   int lines;             // 1: the interior runs the line-staged sweep (sweep_lines.cuh)
   unsigned *err;         // device error word of the handle (a bounded wait gave up)
@@ -161,18 +162,11 @@ struct ReduceArgs {
 
 // ---- launchers (defined in the .cu files, dispatch on lattice and storage) ----
 cudaError_t launch_sweep(int Q, int store, int compute, const SweepArgs &a, cudaStream_t s);
-// Fork/join of the two launches of a channel step: the force kernel runs on
-// `side` while the sweep runs on the main stream (the force kernel only reads
-// the state the sweep reads), joined before anything that follows.
-struct SweepFork {
-  cudaStream_t side;
-  cudaEvent_t fork, join;
-};
 // u, v, w, p of the step that read a.fa (channel profile), into a.mu..a.mp.
 cudaError_t launch_macros_channel(int Q, int store, int compute, const SweepArgs &a,
                                   cudaStream_t s);
 cudaError_t launch_sweep_channel(int Q, int store, int compute, const SweepArgs &a,
-                                 cudaStream_t s, const SweepFork *fk = nullptr);
+                                 cudaStream_t s);
 // Post-stream populations of the step that read a.fa (FP64, dense [i][z][y][x]);
 // ref: plain pull (reference profiles), else the channel's resolved pull.
 cudaError_t launch_stream_state(int Q, int store, const SweepArgs &a, bool ref, double *out,

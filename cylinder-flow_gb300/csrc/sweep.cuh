@@ -625,11 +625,11 @@ __device__ __forceinline__ P pull_pair(const typename Store<ST>::elem *__restric
   else off = I * S - (Dd::ex + Dd::ey * rs + Dd::ez * zs);
   float r0 = 0.0f, r1 = 0.0f;
   if constexpr (Dd::ex < 0) {  // the outlet column repeats itself (pm = p - 1 there)
-    if (act0) r0 = PC::raw(__ldg(pm0 + off));
-    if (act1) r1 = PC::raw(__ldg(pm1 + off));
+    if (act0) r0 = PC::raw(__ldca(pm0 + off));
+    if (act1) r1 = PC::raw(__ldca(pm1 + off));
   } else {
-    if (act0) r0 = PC::raw(__ldg(p + off));
-    if (act1) r1 = PC::raw(__ldg(p + off + 32));
+    if (act0) r0 = PC::raw(__ldca(p + off));
+    if (act1) r1 = PC::raw(__ldca(p + off + 32));
   }
   const float b = a.L.fbase[I];
   float2 v = PC::dec(make_float2(r0, r1), make_float2(b, b));
@@ -649,7 +649,7 @@ __device__ __forceinline__ P pull_pair_listed(const typename Store<ST>::elem *__
   using PC = PairCodec<ST>;
   if constexpr (I == 0) {
     const float b = a.L.fbase[0];
-    return PC::dec(make_float2(PC::raw(__ldg(p)), act1 ? PC::raw(__ldg(p + 32)) : 0.0f),
+    return PC::dec(make_float2(PC::raw(__ldca(p)), act1 ? PC::raw(__ldca(p + 32)) : 0.0f),
                    make_float2(b, b));
   } else {
     const bool bb0 = wbb || ((l0 >> I) & 1u), bb1 = wbb || ((l1 >> I) & 1u);
@@ -661,8 +661,8 @@ __device__ __forceinline__ P pull_pair_listed(const typename Store<ST>::elem *__
     constexpr long long OS = Dd::opp;
     const float b0 = bb0 ? a.L.fbase[Dd::opp] : a.L.fbase[I];
     const float b1 = bb1 ? a.L.fbase[Dd::opp] : a.L.fbase[I];
-    const float r0 = PC::raw(__ldg(p + (bb0 ? a.doff[OS] : s0)));
-    const float r1 = act1 ? PC::raw(__ldg(p + (bb1 ? a.doff[OS] + 32 : s1))) : 0.0f;
+    const float r0 = PC::raw(__ldca(p + (bb0 ? a.doff[OS] : s0)));
+    const float r1 = act1 ? PC::raw(__ldca(p + (bb1 ? a.doff[OS] + 32 : s1))) : 0.0f;
     float2 v = PC::dec(make_float2(r0, r1), make_float2(b0, b1));
     if constexpr (Dd::ex > 0) v.x = (!bb0 && inlet0) ? a.f_in_f[I] : v.x;
     return v;
@@ -758,177 +758,103 @@ __device__ __forceinline__ void channel2_cells(const SweepArgs &a, int x0, int y
                                     (unsigned)(cell0 * Q + i), a.f16_sr);
 }
 
-template <int Q, class ST, class P, int MINB, bool LISTED1 = false>
-__global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB)
-    sweep_channel2_kernel(const SweepArgs a) {
-  const int ny = a.L.ny;
-  const int y = blockIdx.y * SWEEP_BY + threadIdx.y, z = blockIdx.z;
-  if (y >= ny) return;
-  const int w0 = 2 * blockIdx.x;
-  const long long trow = ((long long)z * ny + y) * a.nxw;
-  const bool has1 = w0 + 1 < a.nxw;
-  const int t0 = a.tile_index[trow + w0];
-  const int t1 = has1 ? a.tile_index[trow + w0 + 1] : -1;
-  const int x0 = 32 * w0 + threadIdx.x;
-  // A listed pair returns from its own inlined code: with the packed listed
-  // and plain bodies in an if / else the FP16 kernel spilled 196 bytes, in
-  // this form 60.
-  if (t0 >= 0 || t1 >= 0) {  // warp-uniform
-    const unsigned l0 = t0 >= 0 ? a.links_bits[(long long)t0 * SWEEP_BX + threadIdx.x] : 0u;
-    const unsigned l1 = t1 >= 0 ? a.links_bits[(long long)t1 * SWEEP_BX + threadIdx.x] : 0u;
-    if constexpr (LISTED1) {
-#pragma unroll 1
-      for (int h = 0; h < (has1 ? 2 : 1); ++h)
-        channel_listed_cell<Q, ST, typename PairT<P>::C>(a, x0 + 32 * h, y, z, h ? l1 : l0);
-    } else {
-      channel2_cells<Q, ST, P, true>(a, x0, y, z, true, has1, l0, l1);
-    }
-    return;
-  }
-  channel2_cells<Q, ST, P>(a, x0, y, z, true, has1);
-}
+// Programmatic dependent launch (the one-launch step): a kernel starts while its
+// predecessor on the stream runs; wait() returns when that has finished and its
+// writes are visible.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Channel sweep, one cell per thread, one warp tile per warp, over the whole
-// box: unlisted tiles pull plainly, listed tiles through the face-state tables
-// and their link words (solid cells zeroed).  The tile's listed position is
-// warp-uniform, so is the branch.
-template <int Q, class ST, class A, int MINB>
-__global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_channel_kernel(const SweepArgs a) {
-  using L = Lat<Q>;
-  using SF = Store<ST>;
-  using E = typename SF::elem;
-  const int nx = a.L.nx, ny = a.L.ny;
-  const int lane = threadIdx.x;
-  const int y = blockIdx.y * SWEEP_BY + threadIdx.y, z = blockIdx.z;
-  if (y >= ny) return;
-  const int t = a.tile_index[((long long)z * ny + y) * a.nxw + blockIdx.x];
-  int x = blockIdx.x * SWEEP_BX + lane;
-  const bool valid = x < nx;
-  if (!valid) x = nx - 1;
-  const long long S = a.L.S;
-  const long long c = a.L.idx(x, y, z);
-  const E *__restrict__ fa = static_cast<const E *>(a.fa);
-  E *__restrict__ fb = static_cast<E *>(a.fb);
-  A f[Q];
-  bool solid_here = false;
-  if (t >= 0) {
-    const unsigned links = a.links_bits[(long long)t * SWEEP_BX + lane];
-    solid_here = links >> 31;
-    const int st = face_state(y, z, ny, a.L.nz);
-    const long long *__restrict__ offs = a.face_off + st * Q;
-    const unsigned wbb = a.face_bb[st];
-    static_for(
-        [&](auto ic) {
-          constexpr int I = decltype(ic)::value;
-          f[I] = pull_listed<Q, ST, A, I>(fa, c, S, x, offs[I], (wbb >> I) & 1u, links, a);
-        },
-        std::make_integer_sequence<int, Q>{});
-  } else {
-    static_for(
-        [&](auto ic) {
-          constexpr int I = decltype(ic)::value;
-          f[I] = pull_plain<Q, ST, A, I>(fa, c, S, x, a);
-        },
-        std::make_integer_sequence<int, Q>{});
-  }
-  const long long cell = ((long long)z * ny + y) * nx + x;
-  if constexpr (std::is_same<A, double>::value) {
-    if (fixed_cell<L, SF>(f, solid_here, false, 0.0, false, cell, valid, fb, c, S, a)) return;
-  }
-  A rho3, ux, uy, uz;
-  moments<L, A, SF>(f, rho3, ux, uy, uz);
-  if (solid_here) {
-    rho3 = A(0); ux = A(0); uy = A(0); uz = A(0);
-  }
-  finish_cell<L, SF, A, E>(f, rho3, ux, uy, uz, cell, valid, fb, c, S, a);
-}
-
-// Sums per-thread FP64 force partials of a small grid: warp shuffles, per
-// block into partials[blockIdx.x], then over blocks, in block order, by the last
-// block to finish, into the force-history slot of this step.
+// Sums per-thread FP64 force partials over `nblk` blocks, this one number `blk`:
+// warp shuffles, per block, and over blocks, in block order, by the last block to
+// finish, into the force-history slot of this step.  One block alone needs no
+// partials and no counter.
 __device__ __forceinline__ void force_to_history(const SweepArgs &a, double dx, double dy,
-                                                 double dz) {
+                                                 double dz, unsigned blk, unsigned nblk) {
   constexpr int NW = SWEEP_BY;
   const int lane = threadIdx.x, wid = threadIdx.y;
   const int tid = wid * SWEEP_BX + lane;
   __shared__ double sh[3][NW];
   __shared__ bool last;
-  for (int o = 16; o > 0; o >>= 1) {
-    dx += __shfl_down_sync(0xffffffffu, dx, o);
-    dy += __shfl_down_sync(0xffffffffu, dy, o);
-    dz += __shfl_down_sync(0xffffffffu, dz, o);
+  auto block_sum = [&](double &x, double &y, double &z) {  // valid in thread 0
+    for (int o = 16; o > 0; o >>= 1) {
+      x += __shfl_down_sync(0xffffffffu, x, o);
+      y += __shfl_down_sync(0xffffffffu, y, o);
+      z += __shfl_down_sync(0xffffffffu, z, o);
+    }
+    if (lane == 0) {
+      sh[0][wid] = x;
+      sh[1][wid] = y;
+      sh[2][wid] = z;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      x = y = z = 0.0;
+      for (int w = 0; w < NW; ++w) { x += sh[0][w]; y += sh[1][w]; z += sh[2][w]; }
+    }
+  };
+  auto record = [&] {
+    const long long st = *a.step;
+    double *h = a.hist + 3 * (st % a.cap);
+    h[0] = dx;
+    h[1] = dy;
+    h[2] = dz;
+    *a.step = st + 1;
+  };
+  block_sum(dx, dy, dz);
+  if (nblk == 1) {
+    if (tid == 0) record();
+    return;
   }
-  if (lane == 0) {
-    sh[0][wid] = dx;
-    sh[1][wid] = dy;
-    sh[2][wid] = dz;
-  }
-  __syncthreads();
   if (tid == 0) {
-    double bx = 0.0, by = 0.0, bz = 0.0;
-    for (int w = 0; w < NW; ++w) { bx += sh[0][w]; by += sh[1][w]; bz += sh[2][w]; }
-    a.partials[3 * blockIdx.x] = bx;
-    a.partials[3 * blockIdx.x + 1] = by;
-    a.partials[3 * blockIdx.x + 2] = bz;
+    a.partials[3 * blk] = dx;
+    a.partials[3 * blk + 1] = dy;
+    a.partials[3 * blk + 2] = dz;
     __threadfence();
-    last = atomicAdd(a.counter, 1u) == gridDim.x - 1;
+    last = atomicAdd(a.counter, 1u) == nblk - 1;
   }
   __syncthreads();
   if (last) {
     __threadfence();
     const volatile double *p = a.partials;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    for (unsigned k = tid; k < gridDim.x; k += SWEEP_BX * SWEEP_BY) {
-      s0 += p[3 * k];
-      s1 += p[3 * k + 1];
-      s2 += p[3 * k + 2];
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      s0 += __shfl_down_sync(0xffffffffu, s0, o);
-      s1 += __shfl_down_sync(0xffffffffu, s1, o);
-      s2 += __shfl_down_sync(0xffffffffu, s2, o);
+    dx = dy = dz = 0.0;
+    for (unsigned k = tid; k < nblk; k += SWEEP_BX * SWEEP_BY) {
+      dx += p[3 * k];
+      dy += p[3 * k + 1];
+      dz += p[3 * k + 2];
     }
     __syncthreads();
-    if (lane == 0) {
-      sh[0][wid] = s0;
-      sh[1][wid] = s1;
-      sh[2][wid] = s2;
-    }
-    __syncthreads();
+    block_sum(dx, dy, dz);
     if (tid == 0) {
-      double tx = 0.0, ty = 0.0, tz = 0.0;
-      for (int w = 0; w < NW; ++w) { tx += sh[0][w]; ty += sh[1][w]; tz += sh[2][w]; }
-      const long long st = *a.step;
-      double *h = a.hist + 3 * (st % a.cap);
-      h[0] = tx;
-      h[1] = ty;
-      h[2] = tz;
-      *a.step = st + 1;
+      record();
       *a.counter = 0u;
     }
   }
 }
 
-// Momentum-exchange force on the solids for this step, beside the sweep on a
-// second stream: a small grid (at most one block per SM) strides over the
-// boundary cells (fluid cells with solid links; the set-up's list, in tile and
-// x order), one cell per thread, and reads the populations the sweep bounces
-// back (f*_{opp(I)}(X) from the state it pulls from); per cell the sum runs in
-// the arithmetic type, over cells in FP64.
-template <int Q, class ST, class A, int MINB>
-__global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) channel_force_kernel(const SweepArgs a) {
+// Momentum-exchange force on the solids for this step, by block `blk` of `nblk`:
+// the blocks stride over the boundary cells (fluid cells with solid links; the
+// set-up's list, in tile and x order), one cell per thread, and read the
+// populations the sweep bounces back (f*_{opp(I)}(X) from the state it pulls
+// from); per cell the sum runs in the arithmetic type, over cells in FP64.  PDL:
+// the first cells' list entries are read ahead of the predecessor's end.
+template <int Q, class ST, class A, bool PDL>
+__device__ __forceinline__ void force_cells(const SweepArgs &a, unsigned blk, unsigned nblk) {
   using L = Lat<Q>;
   using SF = Store<ST>;
   using E = typename SF::elem;
   const long long S = a.L.S;
   const E *__restrict__ fa = static_cast<const E *>(a.fa);
-  const long long stride = (long long)gridDim.x * SWEEP_BX * SWEEP_BY;
+  const int stride = (int)nblk * SWEEP_BX * SWEEP_BY;
+  int k = ((int)blk * SWEEP_BY + threadIdx.y) * SWEEP_BX + threadIdx.x;
+  unsigned links = 0;
+  long long c = 0;
+  if (k < a.n_bcells) {
+    links = a.bcell_links[k];
+    c = a.bcell_idx[k];
+  }
+  if constexpr (PDL) pdl_wait();
   double dx = 0.0, dy = 0.0, dz = 0.0;
-  for (long long k = (long long)blockIdx.x * SWEEP_BX * SWEEP_BY + threadIdx.y * SWEEP_BX +
-                     threadIdx.x;
-       k < a.n_bcells; k += stride) {
-    const unsigned links = a.bcell_links[k];
-    const long long c = a.bcell_idx[k];
+  while (k < a.n_bcells) {
     A f[Q];
     static_for(
         [&](auto ic) {
@@ -950,8 +876,129 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) channel_force_kerne
       dy += Fy;
       dz += Fz;
     }
+    k += stride;
+    if (k < a.n_bcells) {
+      links = a.bcell_links[k];
+      c = a.bcell_idx[k];
+    }
   }
-  force_to_history(a, dx, dy, dz);
+  force_to_history(a, dx, dy, dz, blk, nblk);
+}
+
+// The force as a launch of its own: with the line-staged sweep, and where the
+// sweep's grid has no room for its blocks.
+template <int Q, class ST, class A, int MINB>
+__global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) channel_force_kernel(const SweepArgs a) {
+  force_cells<Q, ST, A, false>(a, blockIdx.x, gridDim.x);
+}
+
+// The leading rows (2-D) or planes (3-D) of a sweep's grid form the force.  True when this block was one of them; otherwise by /
+// bz become the sweep's.
+template <int Q, class ST, class A>
+__device__ __forceinline__ bool force_block(const SweepArgs &a, int &by, int &bz) {
+  int &b = Q == 9 ? by : bz;
+  if (b >= a.force_span) {
+    b -= a.force_span;
+    return false;
+  }
+  const unsigned blk = (bz * gridDim.y + by) * gridDim.x + blockIdx.x;
+  if (blk < (unsigned)a.bnd_blocks) force_cells<Q, ST, A, true>(a, blk, a.bnd_blocks);
+  return true;
+}
+
+template <int Q, class ST, class P, int MINB, bool LISTED1 = false>
+__global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB)
+    sweep_channel2_kernel(const SweepArgs a) {
+  const int ny = a.L.ny;
+  int by = blockIdx.y, z = blockIdx.z;
+  pdl_trigger();
+  if (force_block<Q, ST, typename PairT<P>::C>(a, by, z)) return;
+  const int y = by * SWEEP_BY + threadIdx.y;
+  if (y >= ny) return;
+  const int w0 = 2 * blockIdx.x;
+  const long long trow = ((long long)z * ny + y) * a.nxw;
+  const bool has1 = w0 + 1 < a.nxw;
+  const int t0 = a.tile_index[trow + w0];
+  const int t1 = has1 ? a.tile_index[trow + w0 + 1] : -1;
+  const int x0 = 32 * w0 + threadIdx.x;
+  // A listed pair returns from its own inlined code: with the packed listed
+  // and plain bodies in an if / else the FP16 kernel spilled 196 bytes, in
+  // this form 60.
+  if (t0 >= 0 || t1 >= 0) {  // warp-uniform
+    const unsigned l0 = t0 >= 0 ? a.links_bits[(long long)t0 * SWEEP_BX + threadIdx.x] : 0u;
+    const unsigned l1 = t1 >= 0 ? a.links_bits[(long long)t1 * SWEEP_BX + threadIdx.x] : 0u;
+    pdl_wait();
+    if constexpr (LISTED1) {
+#pragma unroll 1
+      for (int h = 0; h < (has1 ? 2 : 1); ++h)
+        channel_listed_cell<Q, ST, typename PairT<P>::C>(a, x0 + 32 * h, y, z, h ? l1 : l0);
+    } else {
+      channel2_cells<Q, ST, P, true>(a, x0, y, z, true, has1, l0, l1);
+    }
+    return;
+  }
+  pdl_wait();
+  channel2_cells<Q, ST, P>(a, x0, y, z, true, has1);
+}
+
+// Channel sweep, one cell per thread, one warp tile per warp, over the whole
+// box: unlisted tiles pull plainly, listed tiles through the face-state tables
+// and their link words (solid cells zeroed).  The tile's listed position is
+// warp-uniform, so is the branch.
+template <int Q, class ST, class A, int MINB>
+__global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_channel_kernel(const SweepArgs a) {
+  using L = Lat<Q>;
+  using SF = Store<ST>;
+  using E = typename SF::elem;
+  const int nx = a.L.nx, ny = a.L.ny;
+  const int lane = threadIdx.x;
+  int by = blockIdx.y, z = blockIdx.z;
+  if (force_block<Q, ST, A>(a, by, z)) return;
+  const int y = by * SWEEP_BY + threadIdx.y;
+  if (y >= ny) return;
+  const int t = a.tile_index[((long long)z * ny + y) * a.nxw + blockIdx.x];
+  int x = blockIdx.x * SWEEP_BX + lane;
+  const bool valid = x < nx;
+  if (!valid) x = nx - 1;
+  const long long S = a.L.S;
+  const long long c = a.L.idx(x, y, z);
+  const E *__restrict__ fa = static_cast<const E *>(a.fa);
+  E *__restrict__ fb = static_cast<E *>(a.fb);
+  A f[Q];
+  bool solid_here = false;
+  if (t >= 0) {
+    const unsigned links = a.links_bits[(long long)t * SWEEP_BX + lane];
+    solid_here = links >> 31;
+    pdl_wait();
+    const int st = face_state(y, z, ny, a.L.nz);
+    const long long *__restrict__ offs = a.face_off + st * Q;
+    const unsigned wbb = a.face_bb[st];
+    static_for(
+        [&](auto ic) {
+          constexpr int I = decltype(ic)::value;
+          f[I] = pull_listed<Q, ST, A, I>(fa, c, S, x, offs[I], (wbb >> I) & 1u, links, a);
+        },
+        std::make_integer_sequence<int, Q>{});
+  } else {
+    pdl_wait();
+    static_for(
+        [&](auto ic) {
+          constexpr int I = decltype(ic)::value;
+          f[I] = pull_plain<Q, ST, A, I>(fa, c, S, x, a);
+        },
+        std::make_integer_sequence<int, Q>{});
+  }
+  const long long cell = ((long long)z * ny + y) * nx + x;
+  pdl_trigger();
+  if constexpr (std::is_same<A, double>::value) {
+    if (fixed_cell<L, SF>(f, solid_here, false, 0.0, false, cell, valid, fb, c, S, a)) return;
+  }
+  A rho3, ux, uy, uz;
+  moments<L, A, SF>(f, rho3, ux, uy, uz);
+  if (solid_here) {
+    rho3 = A(0); ux = A(0); uy = A(0); uz = A(0);
+  }
+  finish_cell<L, SF, A, E>(f, rho3, ux, uy, uz, cell, valid, fb, c, S, a);
 }
 
 // Macroscopic fields of the step that read a.fa, formed on request instead of
@@ -1130,31 +1177,63 @@ cudaError_t launch_macros_channel_t(const SweepArgs &a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// The interior launch: FP32 collision on FP32 or FP16 storage takes the packed
-// two-cells-per-thread kernel; the others the one-cell kernel.
+// One channel step: one launch of the sweep and the force (force_block), started
+// while the previous step still runs (programmatic dependent launch; the kernels
+// read the mask tables ahead of griddepcontrol.wait).  Measured against the sweep
+// with a force launch beside it on a second stream, steps and the fields: D2Q9
+// 1021x241 FP32, 200 steps 0.67 / 0.89 ms, 8192x1024 FP32 1.88 / 1.95 ms; D3Q27
+// 108x52x34 FP32, 100 steps 0.83 / 0.99 ms, 512x128x128 FP32 5.60 / 5.64 ms, FP64
+// 7.98 / 8.07 ms, 768x384x384 FP16 25.7 / 25.7 ms.  The one-cell kernel lets the
+// next step start after its loads: at its start, D2Q9 400x100 FP64 took 6.4 us per
+// step against 4.8 (the waiting blocks' places unbalance the SMs); the pair kernel
+// is better at its start (1021x241: 0.67 against 0.77 ms).
 template <int Q, class ST, class A, int MINB_FAST>
-void launch_interior(const SweepArgs &a, dim3 grid, dim3 block, cudaStream_t s) {
+cudaError_t launch_sweep_channel_t(const SweepArgs &a0, cudaStream_t s) {
+  SweepArgs a = a0;
+  constexpr int TB = SWEEP_BX * SWEEP_BY;
   if constexpr (Q == 27 && sizeof(A) == 4 && std::is_same<ST, F16Dev>::value) {
-    if (a.lines) {  // FP16, ROWS layout: the line-staged sweep
-      (void)launch_lines_f16_q27(a, a.sms, s);
-      return;
+    if (a.lines) {  // FP16, ROWS layout: the line-staged sweep, then the force
+      const cudaError_t e = launch_lines_f16_q27(a, a.sms, s);
+      if (e != cudaSuccess) return e;
+      if (a.bnd_blocks > 0)
+        channel_force_kernel<Q, ST, A, 4><<<a.bnd_blocks, dim3(SWEEP_BX, SWEEP_BY, 1), 0, s>>>(a);
+      count_launch(2);
+      return cudaGetLastError();
     }
   }
-  if constexpr (sizeof(A) == 4 && !std::is_same<ST, double>::value) {
-    // Blocks per SM, measured on the D3Q27 bench step with packed listed
+  constexpr bool pair = sizeof(A) == 4 && !std::is_same<ST, double>::value;
+  dim3 grid(pair ? (a.nxw + 1) / 2 : a.nxw, (a.L.ny + SWEEP_BY - 1) / SWEEP_BY, a.L.nz);
+  // up to 4 boundary cells per thread in one block: its sum needs no partials
+  if (a.bnd_blocks > 1 && a.n_bcells <= 4 * TB) a.bnd_blocks = 1;
+  const int per = (int)(Q == 9 ? grid.x : grid.x * grid.y);
+  a.force_span = (a.bnd_blocks + per - 1) / per;
+  unsigned &span_dim = Q == 9 ? grid.y : grid.z;
+  if (span_dim + a.force_span > 65535u) {  // no room in the grid: a launch of its own
+    channel_force_kernel<Q, ST, A, 4><<<a.bnd_blocks, dim3(SWEEP_BX, SWEEP_BY, 1), 0, s>>>(a);
+    count_launch();
+    a.force_span = 0;
+  }
+  span_dim += a.force_span;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(SWEEP_BX, SWEEP_BY, 1);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  auto launch = [&](auto kernel) { return cudaLaunchKernelEx(&cfg, kernel, a); };
+  cudaError_t e;
+  if constexpr (pair) {
+    // FP32 collision on FP32 or FP16 storage: the packed two-cells-per-thread
+    // kernel.  Blocks per SM, measured on the D3Q27 bench step with packed listed
     // pairs: FP32 storage 0.850 / 0.908 / 0.937 of the copy peak at 4 / 5 / 6
     // per SM (7 and 8 spill more); FP16 0.613 / 0.636 / 0.632.  D2Q9 on grids
     // of 2^20 cells and more: 10 per SM (48 registers; 8192x1024: FP32 storage
     // 0.982 against 0.946 at 6, FP16 0.729 against 0.659); smaller D2Q9 grids
     // are bound by per-thread latency (640x160 FP32: 6.1 us per step at 6
     // against 6.6 at 10).
-    dim3 g2((a.nxw + 1) / 2, grid.y, grid.z);
-    if constexpr (Q == 9) {
-      if ((long long)a.L.nx * a.L.ny * a.L.nz >= (1LL << 20)) {
-        sweep_channel2_kernel<Q, ST, float2, 10><<<g2, block, 0, s>>>(a);
-        return;
-      }
-    }
     // Listed pairs: packed (both cells at once) or one cell after the other
     // (LISTED1; fewer live registers).  One cell at a time, measured on the
     // channel steps: FP16 D3Q27 39.5 against 37.5 G cell updates/s on
@@ -1163,37 +1242,18 @@ void launch_interior(const SweepArgs &a, dim3 grid, dim3 block, cudaStream_t s) 
     // same either way (31.0 / 32.2 at 6 per SM); the wide D2Q9 grids 1-2 %
     // slower (8192x1024: FP16 129.5 against 130.8, FP32 91.4 against 93.3).
     if constexpr (Q == 27 && std::is_same<ST, float>::value)
-      sweep_channel2_kernel<Q, ST, float2, 6><<<g2, block, 0, s>>>(a);
+      e = launch(sweep_channel2_kernel<Q, ST, float2, 6, false>);
+    else if constexpr (Q == 27)
+      e = launch(sweep_channel2_kernel<Q, ST, float2, 5, true>);
     else
-      sweep_channel2_kernel<Q, ST, float2, 5, true><<<g2, block, 0, s>>>(a);
+      e = (long long)a.L.nx * a.L.ny >= (1LL << 20)
+              ? launch(sweep_channel2_kernel<Q, ST, float2, 10, false>)
+              : launch(sweep_channel2_kernel<Q, ST, float2, 5, true>);
   } else {
-    sweep_channel_kernel<Q, ST, A, MINB_FAST><<<grid, block, 0, s>>>(a);
+    e = launch(sweep_channel_kernel<Q, ST, A, MINB_FAST>);
   }
-}
-
-template <int Q, class ST, class A, int MINB_FAST, int MINB_SLOW>
-cudaError_t launch_sweep_channel_t(const SweepArgs &a, cudaStream_t s, const SweepFork *fk) {
-  dim3 block(SWEEP_BX, SWEEP_BY, 1);
-  dim3 grid((a.L.nx + SWEEP_BX - 1) / SWEEP_BX, (a.L.ny + SWEEP_BY - 1) / SWEEP_BY, a.L.nz);
-  const int sb = a.bnd_blocks;
-  if (fk && fk->side) {
-    // The force launch goes first on the (higher-priority) side stream, so its
-    // latency-bound blocks overlap the sweep's streaming.
-    cudaError_t e = cudaEventRecord(fk->fork, s);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(fk->side, fk->fork, 0);
-    if (e != cudaSuccess) return e;
-    channel_force_kernel<Q, ST, A, MINB_SLOW><<<sb > 0 ? sb : 1, block, 0, fk->side>>>(a);
-    e = cudaEventRecord(fk->join, fk->side);
-    if (e != cudaSuccess) return e;
-    launch_interior<Q, ST, A, MINB_FAST>(a, grid, block, s);
-    e = cudaStreamWaitEvent(s, fk->join, 0);
-    if (e != cudaSuccess) return e;
-  } else {
-    launch_interior<Q, ST, A, MINB_FAST>(a, grid, block, s);
-    channel_force_kernel<Q, ST, A, MINB_SLOW><<<sb > 0 ? sb : 1, block, 0, s>>>(a);
-  }
-  count_launch(2);
-  return cudaGetLastError();
+  count_launch();
+  return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 }  // namespace cflbm

@@ -24,20 +24,20 @@ cudaError_t launch_sweep_q27(int store, int compute, const SweepArgs &a, cudaStr
 }
 
 cudaError_t launch_sweep_channel_q27(int store, int compute, const SweepArgs &a,
-                                      cudaStream_t s, const SweepFork *fk) {
+                                      cudaStream_t s) {
   if (compute != COMPUTE_F32) {
     // Block fixed point: 512x128x128, 10 steps and the fields: 9.67 / 8.39 / 8.55 ms
     // at 4 / 5 / 6 per SM; FP64 operations at 3 per SM: 22.78 ms.
     switch (store) {
-      case STORE_F64: return launch_sweep_channel_t<27, double, double, 5, 2>(a, s, fk);
-      case STORE_F32: return launch_sweep_channel_t<27, float, double, 5, 2>(a, s, fk);
-      case STORE_F16: return launch_sweep_channel_t<27, F16Dev, double, 5, 2>(a, s, fk);
+      case STORE_F64: return launch_sweep_channel_t<27, double, double, 5>(a, s);
+      case STORE_F32: return launch_sweep_channel_t<27, float, double, 5>(a, s);
+      case STORE_F16: return launch_sweep_channel_t<27, F16Dev, double, 5>(a, s);
     }
   } else {
     switch (store) {
-      case STORE_F64: return launch_sweep_channel_t<27, double, float, 8, 4>(a, s, fk);
-      case STORE_F32: return launch_sweep_channel_t<27, float, float, 8, 4>(a, s, fk);
-      case STORE_F16: return launch_sweep_channel_t<27, F16Dev, float, 8, 4>(a, s, fk);
+      case STORE_F64: return launch_sweep_channel_t<27, double, float, 8>(a, s);
+      case STORE_F32: return launch_sweep_channel_t<27, float, float, 8>(a, s);
+      case STORE_F16: return launch_sweep_channel_t<27, F16Dev, float, 8>(a, s);
     }
   }
   return cudaErrorInvalidValue;
