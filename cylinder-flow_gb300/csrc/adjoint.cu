@@ -57,6 +57,10 @@ __host__ __device__ constexpr double aw(int i) {
 
 constexpr int ABX = 32, ABY = 4, ANT = ABX * ABY;
 
+// Interior segments from which their units are captured and replayed: a capture
+// and its instantiation cost about what launching a unit 4 times directly does.
+constexpr int GRAPH_UNITS = 8;
+
 constexpr int GMAX = 4;  // contributions per (cell, population) in the adjoint gather
 
 struct AdjArgs {
@@ -67,12 +71,22 @@ struct AdjArgs {
   const uint32_t *mask;            // solid mask (bit-packed)
   int nxw;
   const int *aux;                  // per cell: AUX_SOLID, AUX_REGULAR or irregular entry r
-  const long long *gat;            // per entry: 9 x GMAX dense mu indices (-1: none)
-  const long long *pul;            // per entry: 9 pull sources, s element or -1 - inlet pop
-  const unsigned *lkr;             // per entry: link bits (bit i: source of i is solid)
+  // Per entry, population j's byte (cell_code) at byte j % 4 of word j / 4,
+  // words [..][3][entry]: GMAX contributions to lambda (CODE_NONE: none), and the
+  // pull source (CODE_INLET + p: inlet population p).
+  const unsigned *gat;
+  const unsigned *pul;
+  int nirr;                        // entries
+  const unsigned *lkr;             // per entry: link bits (bit i: source of i is solid), and
+                                   // bit 31 when a population has more than one contribution
   const float *alpha;              // Brinkman porosity or null
   double omega;
   double u_in;
+  // Inlet populations and their derivatives by u_in, formed on the host: in the
+  // kernel their FP64 operations, for one lane of the first column's warps, took
+  // 3 us of the launch (the SMs holding those blocks had their FP64 pipe 98 % busy).
+  double fin[9], dfin[9];
+  float fin_f[9];
   double c_next;                   // objective weight of step t+1 (when seg is null)
   const int *seg;                  // device: index k of the segment being reversed
   const double *c_tab;             // objective weight of every step 0..T+1
@@ -83,15 +97,39 @@ struct AdjArgs {
   double *g_block;                 // per block: [0] omega, [1] u_in (FP64, owned)
 };
 
+// A population p of a cell one step (dx, dy) away (periodic rows wrap), in a byte.
+enum { CODE_INLET = 0xF0, CODE_NONE = 0xFF };
+__device__ __forceinline__ unsigned cell_code(int p, int dx, int dy) {
+  return (unsigned)(p << 4 | (dy + 1) << 2 | (dx + 1));
+}
+
 enum { SRC_CELL = 0, SRC_INLET = 1 };
 enum { AUX_SOLID = -2, AUX_REGULAR = -1 };
+
+// Link bits of cell (x, y): bit i set when the pull of population i meets a solid.
+__device__ __forceinline__ unsigned link_bits(const uint32_t *mask, int nxw, int nx, int ny,
+                                              int wall_y, int x, int y) {
+  unsigned b = 0;
+  for (int i = 1; i < 9; ++i) {
+    int sx = x - AXf(i), sy = y - AYf(i);
+    if (sy < 0 || sy >= ny) {
+      if (wall_y == WALL_PERIODIC) sy = sy < 0 ? sy + ny : sy - ny;
+      else if (wall_y == WALL_FREESLIP) sy = y;
+      else continue;
+    }
+    if (sx < 0) continue;
+    if (sx >= nx) sx = nx - 1;
+    if (mask_solid(mask, nxw, ny, sx, sy, 0)) b |= 1u << i;
+  }
+  return b;
+}
 
 // Pull source of population i at fluid cell (x, y): the forward channel pull
 // for D2Q9 (sweep.cuh, pull_resolved) with the configured y walls.  SRC_CELL:
 // population j of (sx, sy) (bounce-back: the cell's own opposite population).
 // SRC_INLET: inlet equilibrium population j.  lk: the cell's link bits.
-int host_source(int nx, int ny, int wall_y, unsigned lk, int x, int y, int i, int &sx, int &sy,
-                int &j) {
+__device__ __forceinline__ int pull_source(int nx, int ny, int wall_y, unsigned lk, int x, int y,
+                                           int i, int &sx, int &sy, int &j) {
   if (i == 0) {
     sx = x; sy = y; j = 0;
     return SRC_CELL;
@@ -114,61 +152,127 @@ int host_source(int nx, int ny, int wall_y, unsigned lk, int x, int y, int i, in
   return SRC_CELL;
 }
 
-__device__ __forceinline__ double inlet_f(int j, double u) {
+inline double inlet_f(int j, double u) {
   const double e = AXf(j) * u;
   return aw(j) * (3.0 * e + 4.5 * e * e - 1.5 * u * u);
 }
-__device__ __forceinline__ double inlet_dfdu(int j, double u) {
+inline double inlet_dfdu(int j, double u) {
   return aw(j) * (3.0 * AXf(j) + 9.0 * AXf(j) * AXf(j) * u - 3.0 * u);
 }
 
-// Block sums of two FP64 values; the result is valid in thread 0.
-__device__ __forceinline__ void block_sum2(double v0, double v1, double (*sh)[ANT / 32],
-                                           double &o0, double &o1) {
+// Block sum of an FP64 value; valid in thread 0 of the block.
+__device__ __forceinline__ double block_sum(double v, double *sh) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v0 += __shfl_down_sync(0xffffffffu, v0, o);
-    v1 += __shfl_down_sync(0xffffffffu, v1, o);
-  }
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   const int tid = threadIdx.y * ABX + threadIdx.x;
-  if ((tid & 31) == 0) {
-    sh[0][tid >> 5] = v0;
-    sh[1][tid >> 5] = v1;
-  }
   __syncthreads();
-  o0 = o1 = 0.0;
+  if ((tid & 31) == 0) sh[tid >> 5] = v;
+  __syncthreads();
+  double s = 0.0;
   if (tid == 0)
-    for (int w = 0; w < ANT / 32; ++w) {
-      o0 += sh[0][w];
-      o1 += sh[1][w];
-    }
+    for (int w = 0; w < ANT / 32; ++w) s += sh[w];
+  return s;
 }
 
+// Block sum of an FP32 value to FP64 accuracy without the FP64 pipe (two lanes per
+// SM: the shuffle tree of FP64 additions took 4 of the reverse step's 15 us at
+// 1024x256): every value as two integers over the block's largest exponent, 23
+// and 24 bits, whose sums over 128 threads are exact -- 2^-47 of the largest term.
+// Infinities, NaNs and blocks below 2^-86 take the FP64 tree.
+struct IntSums {
+  unsigned top;
+  int hi, lo;
+};
+__device__ __forceinline__ double block_sum(float v, double *sh, IntSums &is) {
+  const int tid = threadIdx.y * ABX + threadIdx.x;
+  // (is was cleared, and a barrier passed, by the caller)
+  const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(v) & 0x7FFFFFFFu);
+  if ((tid & 31) == 0) atomicMax(&is.top, m);
+  __syncthreads();
+  const int e = (int)(is.top >> 23);
+  if (is.top == 0u) return 0.0;
+  if (e < 40 || e == 255) return block_sum((double)v, sh);
+  // |v| < 2^(e - 126): |u| < 2^23
+  const float u = v * __uint_as_float((unsigned)(276 - e) << 23);
+  const int hi = __float2int_rn(u);
+  const int lo = __float2int_rn((u - (float)hi) * 16777216.0f);
+  const int shi = __reduce_add_sync(0xffffffffu, hi), slo = __reduce_add_sync(0xffffffffu, lo);
+  if ((tid & 31) == 0) {
+    atomicAdd(&is.hi, shi);
+    atomicAdd(&is.lo, slo);
+  }
+  __syncthreads();
+  if (tid != 0) return 0.0;
+  return ((double)is.hi + (double)is.lo * (1.0 / 16777216.0)) *
+         __hiloint2double((1023 + e - 149) << 20, 0);
+}
+__device__ __forceinline__ double block_sum(double v, double *sh, IntSums &) {
+  return block_sum(v, sh);
+}
+
+// One reverse step.  Bound by L2 and latency at the differentiation size (1024x256
+// FP32: 124 bytes per cell, 32 MB).
+// Measured, 600 steps of 1024x256 FP32 reversed and recomputed: 11.5 -> 6.5 ms; 10
+// blocks per SM (6 in FP64) against the compiler's choice: 997x252 FP32 8.50 -> 8.44,
+// 380x110 FP64 4.16 -> 4.08 ms for the whole call.
 template <class A, bool FINAL>
-__global__ void __launch_bounds__(ANT) adjoint_kernel(const AdjArgs a) {
-  __shared__ double sh[2][ANT / 32];
+__global__ void __launch_bounds__(ANT, sizeof(A) == 4 ? 10 : 6) adjoint_kernel(const AdjArgs a) {
+  __shared__ double sh[ANT / 32];
+  __shared__ IntSums is;
   const int nx = a.L.nx, ny = a.L.ny;
   const int x = blockIdx.x * ABX + threadIdx.x;
   const int y = blockIdx.y * ABY + threadIdx.y;
   const bool in = x < nx && y < ny;
   const long long N = (long long)nx * ny;
   const long long cell = (long long)y * nx + x;
+  // Ahead of the predecessor's end (programmatic dependent launch): tables only.
+  // Irregular cells take all their indices here, so that their loads are one round
+  // like a regular cell's (reading the lists population by population made the
+  // few irregular warps the whole launch's length: 17 us per step at 1024x256).
   const int aux = in ? a.aux[cell] : AUX_SOLID;
+  unsigned lk = 0u, gw[3], pw[3];
+  if (aux >= 0) {
+    lk = a.lkr[aux];
+#pragma unroll
+    for (int w = 0; w < 3; ++w) {
+      gw[w] = a.gat[(long long)w * a.nirr + aux];
+      if constexpr (!FINAL) pw[w] = a.pul[(long long)w * a.nirr + aux];
+    }
+  }
+  auto code = [](const unsigned *w, int j) { return (w[j / 4] >> (8 * (j % 4))) & 0xFFu; };
+  // dense index of a contribution, storage index of a source
+  auto row = [&](unsigned c) {
+    int yy = y + (int)((c >> 2) & 3u) - 1;
+    return yy < 0 ? yy + ny : yy >= ny ? yy - ny : yy;
+  };
+  auto dense = [&](unsigned c) {
+    return (long long)(c >> 4) * N + (long long)row(c) * nx + x + (int)(c & 3u) - 1;
+  };
+  auto stored = [&](unsigned c) {
+    return (long long)(c >> 4) * a.L.S + a.L.idx(x + (int)(c & 3u) - 1, row(c), 0);
+  };
+  A al = A(0);
+  if constexpr (!FINAL)
+    if (a.alpha && aux != AUX_SOLID) al = A(a.alpha[cell]);
+  if (threadIdx.x == 0 && threadIdx.y == 0) is = {0u, 0, 0};
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const A *mu_n = static_cast<const A *>(a.mu_next);
   const A *s = static_cast<const A *>(a.s);
   A *ga = static_cast<A *>(a.g_alpha);
-  double d_omega = 0.0, d_u = 0.0;
 
   // lambda_{t+1}(X) = (P^T mu^{t+2})(X) + c_{t+1} dF/ds_{t+1}(X), and (not FINAL)
   // g_{t+1}(X) = (P s_t)(X).  Regular cells: plain shifts.  Irregular cells (box
-  // faces, next to the body): the host-built lists of contributing (Y, i) and of
-  // pull sources.  Every load of a path is issued before any is used.
+  // faces, next to the body): the lists of contributing (Y, i) and of pull sources.
+  // Every load of a path is issued before any is used.
   A lam[9], g[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) lam[k] = g[k] = A(0);
-  A al = A(0), gacc = A(0);
-  int inl = 0;       // bit i: population i of g comes from the inlet
-  long long pe[9];   // irregular: pull sources (inlet: -1 - population)
+  A gacc = A(0);
+  double *gb = a.g_block + 2 * ((long long)blockIdx.y * gridDim.x + blockIdx.x);
+  double gb0 = 0.0;
+  if constexpr (!FINAL)
+    if (threadIdx.x == 0 && threadIdx.y == 0) gb0 = gb[0];
+  int inl = 0;  // bit i: population i of g comes from the inlet
   if (aux == AUX_REGULAR) {
 #pragma unroll
     for (int j = 0; j < 9; ++j) lam[j] = mu_n[j * N + cell + (long long)AYf(j) * nx + AXf(j)];
@@ -176,47 +280,56 @@ __global__ void __launch_bounds__(ANT) adjoint_kernel(const AdjArgs a) {
       const long long c = a.L.idx(x, y, 0);
 #pragma unroll
       for (int i = 0; i < 9; ++i) g[i] = s[i * a.L.S + c - a.L.off(AXf(i), AYf(i), 0)];
-      if (a.alpha) al = A(a.alpha[cell]);
       gacc = ga[cell];
     }
   } else if (aux >= 0) {
-    const long long *gt = a.gat + (long long)aux * 9 * GMAX;
-    long long ge[9 * GMAX];
 #pragma unroll
-    for (int k = 0; k < 9 * GMAX; ++k) ge[k] = gt[k];
-    const unsigned lk = a.lkr[aux];
-    if constexpr (!FINAL) {
-#pragma unroll
-      for (int i = 0; i < 9; ++i) pe[i] = a.pul[(long long)aux * 9 + i];
+    for (int j = 0; j < 9; ++j) {
+      const unsigned c = code(gw, j);
+      if (c != CODE_NONE) lam[j] = mu_n[dense(c)];
     }
-#pragma unroll
-    for (int j = 0; j < 9; ++j)
-#pragma unroll
-      for (int m = 0; m < GMAX; ++m)
-        if (ge[j * GMAX + m] >= 0) lam[j] += mu_n[ge[j * GMAX + m]];
     if constexpr (!FINAL) {
 #pragma unroll
       for (int i = 0; i < 9; ++i) {
-        if (pe[i] >= 0) {
-          g[i] = s[pe[i]];
-        } else {
-          g[i] = A(inlet_f((int)(-1 - pe[i]), a.u_in));
+        const unsigned c = code(pw, i);
+        if (c < CODE_INLET) g[i] = s[stored(c)];
+      }
+      gacc = ga[cell];
+#pragma unroll
+      for (int i = 0; i < 9; ++i) {
+        const unsigned c = code(pw, i);
+        if (c >= CODE_INLET) {
+          if constexpr (sizeof(A) == 4) g[i] = a.fin_f[c - CODE_INLET];
+          else g[i] = a.fin[c - CODE_INLET];
           inl |= 1 << i;
         }
       }
-      if (a.alpha) al = A(a.alpha[cell]);
-      gacc = ga[cell];
     }
+    if (lk >> 31)  // further contributions
+      for (int m = 1; m < GMAX; ++m) {
+#pragma unroll
+        for (int w = 0; w < 3; ++w) gw[w] = a.gat[(long long)(3 * m + w) * a.nirr + aux];
+#pragma unroll
+        for (int j = 0; j < 9; ++j) {
+          const unsigned c = code(gw, j);
+          if (c != CODE_NONE) lam[j] += mu_n[dense(c)];
+        }
+      }
+    lk &= 0x7FFFFFFFu;
     if (lk) {
       // The segment index lives on the device so one captured graph reverses any
       // full segment: a launch reads k and the weight of its step t + 1.
-      const double c_next = a.seg ? a.c_tab[(long long)(*a.seg) * a.K + 2 + a.q] : a.c_next;
+      const A c2 =
+          A(2.0 * (a.seg ? a.c_tab[(long long)(*a.seg) * a.K + 2 + a.q] : a.c_next));
 #pragma unroll
       for (int j = 1; j < 9; ++j)
-        if ((lk >> AOPPf(j)) & 1u)
-          lam[j] += A(c_next * 2.0 * (a.obj_axis == 0 ? AXf(j) : AYf(j)));
+        if ((lk >> AOPPf(j)) & 1u) {
+          const int e = a.obj_axis == 0 ? AXf(j) : AYf(j);
+          if (e != 0) lam[j] += e > 0 ? c2 : -c2;
+        }
     }
   }
+  asm volatile("griddepcontrol.launch_dependents;");
   if constexpr (FINAL) {
     if (in) {
 #pragma unroll
@@ -224,63 +337,116 @@ __global__ void __launch_bounds__(ANT) adjoint_kernel(const AdjArgs a) {
     }
     return;
   } else {
-    A mu[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) mu[k] = A(0);
+    double d_u = 0.0;
+    A dom = A(0);
     if (aux != AUX_SOLID) {
       // ---- mu = C'(g)^T lambda and the collision sensitivities -------------------
-      A rho3 = A(0), jx = A(0), jy = A(0);
+      const A one_a = A(1) - al, om = A(a.omega);
+      A mu[9], jx, jy, vx, vy;
+      if constexpr (sizeof(A) == 4) {
+        // Population by population.  (Written with the forward sweep's conserving
+        // constants the FP32 gradients come out 4 to 8 times nearer to FP64 on most
+        // fields, but further off on the few where the rounding of the weights
+        // happens to cancel the forward run's.)
+        A rho3 = A(0);
+        jx = jy = A(0);
 #pragma unroll
-      for (int i = 0; i < 9; ++i) {
-        rho3 += g[i];
-        jx += g[i] * A(AXf(i));
-        jy += g[i] * A(AYf(i));
+        for (int i = 0; i < 9; ++i) {
+          rho3 += g[i];
+          if (AXf(i) != 0) jx += AXf(i) > 0 ? g[i] : -g[i];
+          if (AYf(i) != 0) jy += AYf(i) > 0 ? g[i] : -g[i];
+        }
+        const A bx = one_a * jx, by = one_a * jy;
+        const A usq = bx * bx + by * by;
+        A A0 = A(0), A1x = A(0), A1y = A(0), A2x = A(0), A2y = A(0);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+          const A w = A(aw(k));
+          const A ex = AXf(k) == 0 ? A(0) : AXf(k) > 0 ? bx : -bx;
+          const A ey = AYf(k) == 0 ? A(0) : AYf(k) > 0 ? by : -by;
+          const A eu = AXf(k) == 0 ? ey : AYf(k) == 0 ? ex : ex + ey;
+          const A feq = k == 0 ? w * (rho3 - A(1.5) * usq)
+                               : w * (rho3 + A(3) * eu + A(4.5) * eu * eu - A(1.5) * usq);
+          dom += lam[k] * (feq - g[k]);
+          const A lw = lam[k] * w, lwe = lw * eu;
+          A0 += lw;
+          if (AXf(k) != 0) {
+            A1x += AXf(k) > 0 ? lw : -lw;
+            A2x += AXf(k) > 0 ? lwe : -lwe;
+          }
+          if (AYf(k) != 0) {
+            A1y += AYf(k) > 0 ? lw : -lw;
+            A2y += AYf(k) > 0 ? lwe : -lwe;
+          }
+        }
+        vx = A(3) * A1x + A(9) * A2x - A(3) * bx * A0;
+        vy = A(3) * A1y + A(9) * A2y - A(3) * by * A0;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+          const A px = AXf(i) == 0 ? A(0) : AXf(i) > 0 ? vx : -vx;
+          const A py = AYf(i) == 0 ? A(0) : AYf(i) > 0 ? vy : -vy;
+          const A ve = AXf(i) == 0 ? py : AYf(i) == 0 ? px : px + py;
+          mu[i] = (A(1) - om) * lam[i] + om * (i == 0 ? A0 : A0 + one_a * ve);
+        }
+      } else {
+        // Over the +/- pairs: 130 FP64 operations, the pipe that binds here, for 310.
+        constexpr A w0 = A(4.0 / 9.0), w1 = A(1.0 / 9.0), w2 = A(1.0 / 36.0);
+        const A rho3 = g[0] + ((g[1] + g[3]) + (g[2] + g[4])) + ((g[5] + g[7]) + (g[6] + g[8]));
+        jx = (g[1] - g[3]) + ((g[5] - g[7]) + (g[8] - g[6]));
+        jy = (g[2] - g[4]) + ((g[5] - g[7]) + (g[6] - g[8]));
+        const A bx = one_a * jx, by = one_a * jy;
+        const A c0 = rho3 - A(1.5) * (bx * bx + by * by);
+        const A bp = bx + by, bm = by - bx;  // e.u of populations 5 and 6
+        dom = lam[0] * (w0 * c0 - g[0]);
+        auto pair = [&](int i, int j, A w, A eu) {  // lambda (feq - g) of i and its opposite j
+          const A ev = c0 + A(4.5) * (eu * eu);
+          dom += lam[i] * (w * (ev + A(3) * eu) - g[i]);
+          dom += lam[j] * (w * (ev - A(3) * eu) - g[j]);
+        };
+        pair(1, 3, w1, bx);
+        pair(2, 4, w1, by);
+        pair(5, 7, w2, bp);
+        pair(6, 8, w2, bm);
+        const A s1 = lam[1] + lam[3], s2 = lam[2] + lam[4], s5 = lam[5] + lam[7],
+                s6 = lam[6] + lam[8];
+        const A d1 = lam[1] - lam[3], d2 = lam[2] - lam[4], d5 = lam[5] - lam[7],
+                d6 = lam[6] - lam[8];
+        const A A0 = w0 * lam[0] + w1 * (s1 + s2) + w2 * (s5 + s6);
+        const A A1x = w1 * d1 + w2 * (d5 - d6), A1y = w1 * d2 + w2 * (d5 + d6);
+        const A A2x = w1 * (s1 * bx) + w2 * (s5 * bp - s6 * bm);
+        const A A2y = w1 * (s2 * by) + w2 * (s5 * bp + s6 * bm);
+        vx = A(3) * A1x + A(9) * A2x - A(3) * (bx * A0);
+        vy = A(3) * A1y + A(9) * A2y - A(3) * (by * A0);
+        const A omc = A(1) - om, P = om * A0, qx = om * (one_a * vx), qy = om * (one_a * vy);
+        const A qp = qx + qy, qm = qy - qx;
+        const A add[9] = {P, P + qx, P + qy, P - qx, P - qy, P + qp, P + qm, P - qp, P - qm};
+#pragma unroll
+        for (int i = 0; i < 9; ++i) mu[i] = omc * lam[i] + add[i];
       }
-      const A one_a = A(1) - al;
-      const A bx = one_a * jx, by = one_a * jy;
-      const A om = A(a.omega);
-      const A usq = bx * bx + by * by;
-      A A0 = A(0), A1x = A(0), A1y = A(0), A2x = A(0), A2y = A(0), dom = A(0);
-#pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        const A w = A(aw(k));
-        const A eu = A(AXf(k)) * bx + A(AYf(k)) * by;
-        const A feq = w * (rho3 + A(3) * eu + A(4.5) * eu * eu - A(1.5) * usq);
-        dom += lam[k] * (feq - g[k]);
-        const A lw = lam[k] * w;
-        A0 += lw;
-        A1x += lw * A(AXf(k));
-        A1y += lw * A(AYf(k));
-        A2x += lw * eu * A(AXf(k));
-        A2y += lw * eu * A(AYf(k));
-      }
-      const A vx = A(3) * A1x + A(9) * A2x - A(3) * bx * A0;
-      const A vy = A(3) * A1y + A(9) * A2y - A(3) * by * A0;
-#pragma unroll
-      for (int i = 0; i < 9; ++i)
-        mu[i] = (A(1) - om) * lam[i] + om * (A0 + one_a * (vx * A(AXf(i)) + vy * A(AYf(i))));
       if (inl) {
 #pragma unroll
         for (int i = 0; i < 9; ++i)
           if ((inl >> i) & 1)
-            d_u += static_cast<double>(mu[i]) * inlet_dfdu((int)(-1 - pe[i]), a.u_in);
+            d_u += static_cast<double>(mu[i]) *
+                   a.dfin[code(pw, i) - CODE_INLET];
       }
       // d feq / d alpha, with d u_B / d alpha = -(jx, jy).
-      const A dal = om * (-A(3) * (A1x * jx + A1y * jy) - A(9) * (A2x * jx + A2y * jy) +
-                          A(3) * (bx * jx + by * jy) * A0);
-      ga[cell] = gacc + dal;
-      d_omega = static_cast<double>(dom);
-    }
-    if (in) {
+      ga[cell] = gacc - om * (vx * jx + vy * jy);
 #pragma unroll
       for (int k = 0; k < 9; ++k) static_cast<A *>(a.mu_out)[k * N + cell] = mu[k];
     }
-    double so, su;
-    block_sum2(d_omega, d_u, sh, so, su);
+    // the inlet is the column x = 0: lane 0 of a warp
+    __shared__ double shu[ABY];
+    if (x == 0) shu[threadIdx.y] = d_u;
+    __syncthreads();
+    const double so = block_sum(dom, sh, is);
     if (threadIdx.x == 0 && threadIdx.y == 0) {
-      double *gb = a.g_block + 2 * ((long long)blockIdx.y * gridDim.x + blockIdx.x);
-      gb[0] += so;
-      gb[1] += su;
+      gb[0] = gb0 + so;
+      if (x == 0) {
+        double su = 0.0;
+        for (int w = 0; w < ABY; ++w) su += shu[w];
+        gb[1] += su;
+      }
     }
   }
 }
@@ -289,8 +455,9 @@ __global__ void __launch_bounds__(ANT) adjoint_kernel(const AdjArgs a) {
 // U0 = (u_in, v0) in fluid cells, U_B = (1 - alpha) U0, p = 0.
 template <class A>
 __global__ void __launch_bounds__(ANT) init_sens_kernel(const AdjArgs a, const A *lam1,
-                                                        const double *v0, double *g_alpha64) {
-  __shared__ double sh[2][ANT / 32];
+                                                        unsigned long long seed, double amp,
+                                                        double *g_alpha64) {
+  __shared__ double sh[ANT / 32];
   const int nx = a.L.nx, ny = a.L.ny;
   const int x = blockIdx.x * ABX + threadIdx.x;
   const int y = blockIdx.y * ABY + threadIdx.y;
@@ -299,7 +466,7 @@ __global__ void __launch_bounds__(ANT) init_sens_kernel(const AdjArgs a, const A
   double gu = 0.0, gom = 0.0;
   if (x < nx && y < ny && !mask_solid(a.mask, a.nxw, ny, x, y, 0)) {
     const double al = a.alpha ? (double)a.alpha[cell] : 0.0;
-    const double ux = a.u_in, uy = v0[cell];
+    const double ux = a.u_in, uy = perturbation(seed, cell, amp);
     const double bx = (1.0 - al) * ux, by = (1.0 - al) * uy;
     const double om = a.omega;
     double gal = 0.0;
@@ -317,8 +484,7 @@ __global__ void __launch_bounds__(ANT) init_sens_kernel(const AdjArgs a, const A
     }
     g_alpha64[cell] += gal;
   }
-  double so, su;
-  block_sum2(gom, gu, sh, so, su);
+  const double so = block_sum(gom, sh), su = block_sum(gu, sh);
   if (threadIdx.x == 0 && threadIdx.y == 0) {
     double *gb = a.g_block + 2 * ((long long)blockIdx.y * gridDim.x + blockIdx.x);
     gb[0] += so;
@@ -359,19 +525,28 @@ int afail(int code, const std::string &m) { return record_error(code, m.c_str())
       return afail(CFLBM_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));     \
   } while (0)
 
-// Device scratch of one adjoint run, freed on return.
+// Device scratch of one adjoint run: arrays laid out in one allocation, freed on
+// return.
 struct AdjScratch {
-  std::vector<void *> ptrs;
+  char *base = nullptr;
+  size_t bytes = 0;
+  std::vector<std::pair<void **, size_t>> parts;
   ~AdjScratch() {
-    for (void *p : ptrs) cudaFree(p);
+    if (base) cudaFree(base);
   }
   template <class T>
-  cudaError_t alloc(T **p, size_t n) {
-    void *v = nullptr;
-    cudaError_t e = cudaMalloc(&v, std::max<size_t>(n, 1) * sizeof(T));
-    if (e == cudaSuccess) ptrs.push_back(v);
-    *p = static_cast<T *>(v);
-    return e;
+  void add(T **p, size_t n) {
+    parts.push_back({reinterpret_cast<void **>(p), bytes});
+    bytes += (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
+  }
+  cudaError_t alloc() {
+    const cudaError_t e = cudaMalloc(&base, bytes);
+    if (e != cudaSuccess) {
+      base = nullptr;
+      return e;
+    }
+    for (const auto &p : parts) *p.first = base + p.second;
+    return cudaSuccess;
   }
 };
 
@@ -393,90 +568,88 @@ struct AdjStreams {
   }
 };
 
-// Host tables of the reverse sweep.  Every fluid cell X is classified from the
-// forward pull itself: X is regular when its own pull is the plain shift
-// (source X - e_i, population i, for every i) and the pulls that read X are
-// exactly the 9 plain ones ((X + e_j, j) for every j).  For every other fluid
-// cell (box faces, cells next to the body) the entry lists, per population j of
-// X, the dense mu indices i*N + Y of every pull (Y, i) whose source is (X, j),
-// and X's own 9 pull sources; lk holds its link bits (the momentum-exchange
-// force reads them).
-struct AdjTables {
-  std::vector<int> aux;
-  std::vector<long long> gat, pul;
-  std::vector<unsigned> lkr;
-};
+// Tables of the reverse sweep.  Every fluid cell X is classified from the forward
+// pull itself: X is regular when its own pull is the plain shift (source X - e_i,
+// population i, for every i) and the pulls that read X are exactly the 9 plain ones
+// ((X + e_j, j) for every j) -- away from the box's faces, all 8 neighbours fluid.
+// For every other fluid cell (box faces, cells next to the body) the entry lists,
+// per population j of X, every pull (Y, i) whose source is (X, j), in the order of
+// (Y, i), and X's own 9 pull sources; lkr holds its
+// link bits (the momentum-exchange force reads them).  Entries are numbered as they
+// come; counters: [0] entries, [1] more than GMAX pulls read one population.
+__global__ void __launch_bounds__(ANT) classify_kernel(const uint32_t *mask, int nxw, int nx,
+                                                       int ny, int *aux, int *counters) {
+  const int x = blockIdx.x * ABX + threadIdx.x, y = blockIdx.y * ABY + threadIdx.y;
+  if (x >= nx || y >= ny) return;
+  int v = AUX_REGULAR;
+  if (mask_solid(mask, nxw, ny, x, y, 0)) {
+    v = AUX_SOLID;
+  } else {
+    bool irr = x == 0 || x == nx - 1 || y == 0 || y == ny - 1;
+    for (int d = 0; d < 9 && !irr; ++d)
+      irr = mask_solid(mask, nxw, ny, x + d % 3 - 1, y + d / 3 - 1, 0);
+    if (irr) v = atomicAdd(&counters[0], 1);
+  }
+  aux[(long long)y * nx + x] = v;
+}
 
-int adjoint_tables(const cflbm_handle *h, const std::vector<uint8_t> &solid, AdjTables &t) {
-  const int nx = h->L.nx, ny = h->L.ny, wall = h->cfg.wall_y;
-  const long long N = (long long)nx * ny;
-  std::vector<unsigned> lk((size_t)N, 0u);
-  for (int y = 0; y < ny; ++y)
-    for (int x = 0; x < nx; ++x) {
-      unsigned b = 0;
-      for (int i = 1; i < 9; ++i) {
-        int sx = x - AXf(i), sy = y - AYf(i);
-        if (sy < 0 || sy >= ny) {
-          if (wall == CFLBM_WALL_PERIODIC) sy = (sy + ny) % ny;
-          else if (wall == CFLBM_WALL_FREESLIP) sy = y;
-          else continue;
-        }
-        if (sx < 0) continue;
-        if (sx >= nx) sx = nx - 1;
-        if (solid[(size_t)sy * nx + sx]) b |= 1u << i;
-      }
-      lk[(size_t)y * nx + x] = b;
+__global__ void __launch_bounds__(ANT) tables_kernel(const Layout L, const uint32_t *mask,
+                                                     int nxw, int wall_y, const int *aux,
+                                                     long long nirr, unsigned *gat,
+                                                     unsigned *pul, unsigned *lkr,
+                                                     int *counters) {
+  const int nx = L.nx, ny = L.ny;
+  const int x = blockIdx.x * ABX + threadIdx.x, y = blockIdx.y * ABY + threadIdx.y;
+  if (x >= nx || y >= ny) return;
+  const int r = aux[(long long)y * nx + x];
+  if (r < 0) return;
+  const unsigned lk = link_bits(mask, nxw, nx, ny, wall_y, x, y);
+  // (x, y) -> (xx, yy) in steps; a wrapped row is one step the other way
+  auto step_y = [&](int yy) { return yy == y ? 0 : (yy == y + 1 || yy == y + 1 - ny) ? 1 : -1; };
+  unsigned w[3] = {0u, 0u, 0u};
+  for (int i = 0; i < 9; ++i) {
+    int sx, sy, j;
+    const int kind = pull_source(nx, ny, wall_y, lk, x, y, i, sx, sy, j);
+    const unsigned c = kind == SRC_INLET ? CODE_INLET + j : cell_code(j, sx - x, step_y(sy));
+    w[i / 4] |= c << (8 * (i % 4));
+  }
+  for (int k = 0; k < 3; ++k) pul[k * nirr + r] = w[k];
+  unsigned gw[3 * GMAX];
+  for (int k = 0; k < 3 * GMAX; ++k) gw[k] = ~0u;  // CODE_NONE
+  int cnt[9] = {0};
+  // the neighbouring rows in ascending order (periodic walls wrap)
+  int rows[3], nr = 0;
+  for (int d = -1; d <= 1; ++d) {
+    int yy = y + d;
+    if (yy < 0 || yy >= ny) {
+      if (wall_y != WALL_PERIODIC) continue;
+      yy = yy < 0 ? yy + ny : yy - ny;
     }
-  std::vector<uint8_t> plain((size_t)N, 0), bad((size_t)N, 0);
-  for (int y = 0; y < ny; ++y)
-    for (int x = 0; x < nx; ++x) {
-      const size_t Y = (size_t)y * nx + x;
-      if (solid[Y]) continue;
+    int at = nr++;
+    for (; at > 0 && rows[at - 1] > yy; --at) rows[at] = rows[at - 1];
+    rows[at] = yy;
+  }
+  for (int k = 0; k < nr; ++k)
+    for (int xx = max(x - 1, 0); xx <= min(x + 1, nx - 1); ++xx) {
+      const int yy = rows[k];
+      if (mask_solid(mask, nxw, ny, xx, yy, 0)) continue;
+      const unsigned lY = link_bits(mask, nxw, nx, ny, wall_y, xx, yy);
       for (int i = 0; i < 9; ++i) {
         int sx, sy, j;
-        if (host_source(nx, ny, wall, lk[Y], x, y, i, sx, sy, j) == SRC_INLET) {
-          bad[Y] = 1;
+        if (pull_source(nx, ny, wall_y, lY, xx, yy, i, sx, sy, j) == SRC_INLET || sx != x || sy != y)
+          continue;
+        if (cnt[j] == GMAX) {
+          counters[1] = 1;
           continue;
         }
-        const bool shift = sx == x - AXf(i) && sy == y - AYf(i) && j == i;
-        if (!shift) bad[Y] = 1;
-        const size_t X = (size_t)sy * nx + sx;
-        if (shift) ++plain[X];
-        else bad[X] = 1;
+        const unsigned c = cell_code(i, xx - x, step_y(yy)) ^ 0xFFu;
+        gw[3 * cnt[j]++ + j / 4] ^= c << (8 * (j % 4));
       }
     }
-  t.aux.assign((size_t)N, AUX_REGULAR);
-  long long nirr = 0;
-  for (size_t c = 0; c < (size_t)N; ++c) {
-    if (solid[c]) t.aux[c] = AUX_SOLID;
-    else if (bad[c] || plain[c] != 9) t.aux[c] = (int)nirr++;
-  }
-  t.gat.assign((size_t)nirr * 9 * GMAX, -1);
-  t.pul.assign((size_t)nirr * 9, 0);
-  t.lkr.assign((size_t)nirr, 0u);
-  for (int y = 0; y < ny; ++y)
-    for (int x = 0; x < nx; ++x) {
-      const size_t Y = (size_t)y * nx + x;
-      if (solid[Y]) continue;
-      const int rY = t.aux[Y];
-      if (rY >= 0) t.lkr[rY] = lk[Y];
-      for (int i = 0; i < 9; ++i) {
-        int sx, sy, j;
-        const int kind = host_source(nx, ny, wall, lk[Y], x, y, i, sx, sy, j);
-        if (rY >= 0)
-          t.pul[(size_t)rY * 9 + i] = kind == SRC_INLET ? -1 - j : j * h->L.S + h->L.idx(sx, sy, 0);
-        if (kind == SRC_INLET) continue;
-        const int rX = t.aux[(size_t)sy * nx + sx];
-        if (rX < 0) continue;
-        long long *slot = &t.gat[((size_t)rX * 9 + j) * GMAX];
-        int m = 0;
-        while (m < GMAX && slot[m] >= 0) ++m;
-        if (m == GMAX)
-          return afail(CFLBM_E_UNSUPPORTED, "cflbm_adjoint: more than 4 pulls read one population");
-        slot[m] = (long long)i * N + (long long)Y;
-      }
-    }
-  return CFLBM_OK;
+  for (int k = 0; k < 3 * GMAX; ++k) gat[k * nirr + r] = gw[k];
+  bool more = false;
+  for (int j = 0; j < 9; ++j) more = more || cnt[j] > 1;
+  lkr[r] = lk | (more ? 0x80000000u : 0u);
 }
 
 template <class A>
@@ -496,58 +669,44 @@ int run_adjoint(cflbm_handle *h, const cflbm_adjoint_spec *sp, double *dJ_dalpha
   AdjScratch sc;
   char *ck = nullptr, *seg = nullptr;
   A *mu0 = nullptr, *mu1 = nullptr, *ga = nullptr;
-  double *ga64 = nullptr, *gblk = nullptr, *v0 = nullptr;
-  int *aux = nullptr;
-  long long *gat = nullptr, *pul = nullptr;
-  unsigned *lkr = nullptr;
-  double *scr_part = nullptr, *scr_hist = nullptr;
-  unsigned *scr_cnt = nullptr;
-  long long *scr_step = nullptr;
-  ACK(sc.alloc(&ck, (size_t)nck * sb));
-  ACK(sc.alloc(&seg, 2 * (size_t)K * sb));
-  ACK(sc.alloc(&mu0, 9 * (size_t)N));
-  ACK(sc.alloc(&mu1, 9 * (size_t)N));
-  ACK(sc.alloc(&ga, N));
-  ACK(sc.alloc(&ga64, N));
-  ACK(sc.alloc(&gblk, 2 * nblk));
-  ACK(sc.alloc(&v0, N));
-  ACK(sc.alloc(&aux, N));
-  ACK(sc.alloc(&scr_part, 3 * (size_t)(h->n_slow + 4)));
-  ACK(sc.alloc(&scr_hist, 3));
-  ACK(sc.alloc(&scr_cnt, 1));
-  ACK(sc.alloc(&scr_step, 1));
-  ACK(cudaMemsetAsync(mu1, 0, 9 * N * sizeof(A), st));
-  ACK(cudaMemsetAsync(ga, 0, N * sizeof(A), st));
-  ACK(cudaMemsetAsync(ga64, 0, N * 8, st));
-  ACK(cudaMemsetAsync(gblk, 0, 2 * nblk * 8, st));
-  ACK(cudaMemsetAsync(scr_cnt, 0, 4, st));
-  ACK(cudaMemsetAsync(scr_step, 0, 8, st));
-  long long n_irregular = 0;
-  {
-    std::vector<uint32_t> mw((size_t)h->nxw * ny);
-    ACK(cudaMemcpyAsync(mw.data(), h->d_mask, mw.size() * 4, cudaMemcpyDeviceToHost, st));
-    ACK(cudaStreamSynchronize(st));
-    std::vector<uint8_t> solid(N);
-    for (int y = 0; y < ny; ++y)
-      for (int x = 0; x < nx; ++x)
-        solid[(size_t)y * nx + x] = (mw[(size_t)y * h->nxw + (x >> 5)] >> (x & 31)) & 1u;
-    AdjTables tb;
-    int trc = adjoint_tables(h, solid, tb);
-    if (trc) return trc;
-    n_irregular = (long long)tb.lkr.size();
-    ACK(sc.alloc(&gat, tb.gat.size()));
-    ACK(sc.alloc(&pul, tb.pul.size()));
-    ACK(sc.alloc(&lkr, tb.lkr.size()));
-    std::vector<double> pv(N);
-    for (long long n = 0; n < N; ++n)
-      pv[n] = solid[n] ? 0.0 : perturbation(h->cfg.seed, n, h->cfg.perturb_amp);
-    ACK(cudaMemcpyAsync(aux, tb.aux.data(), N * 4, cudaMemcpyHostToDevice, st));
-    ACK(cudaMemcpyAsync(gat, tb.gat.data(), tb.gat.size() * 8, cudaMemcpyHostToDevice, st));
-    ACK(cudaMemcpyAsync(pul, tb.pul.data(), tb.pul.size() * 8, cudaMemcpyHostToDevice, st));
-    ACK(cudaMemcpyAsync(lkr, tb.lkr.data(), tb.lkr.size() * 4, cudaMemcpyHostToDevice, st));
-    ACK(cudaMemcpyAsync(v0, pv.data(), N * 8, cudaMemcpyHostToDevice, st));
-    ACK(cudaStreamSynchronize(st));
-  }
+  double *ga64 = nullptr, *gblk = nullptr, *c_tab = nullptr;
+  int *aux = nullptr, *counters = nullptr, *d_seg = nullptr;
+  unsigned *gat = nullptr, *pul = nullptr, *lkr = nullptr;
+  // One block for all (a cudaMalloc and its cudaFree cost about 0.1 ms each).  What
+  // starts at zero comes first: mu1, ga, ga64, gblk, counters.
+  sc.add(&mu1, 9 * (size_t)N);
+  sc.add(&ga, N);
+  sc.add(&ga64, N);
+  sc.add(&gblk, 2 * nblk);
+  sc.add(&counters, 2);
+  const size_t zeroed = sc.bytes;
+  sc.add(&mu0, 9 * (size_t)N);
+  sc.add(&aux, N);
+  sc.add(&d_seg, 2);
+  sc.add(&c_tab, (size_t)T + 2);
+  sc.add(&ck, (size_t)nck * sb);
+  sc.add(&seg, 2 * (size_t)K * sb);
+  ACK(sc.alloc());
+  ACK(cudaMemsetAsync(sc.base, 0, zeroed, st));
+  classify_kernel<<<grd, blk, 0, st>>>(h->d_mask, h->nxw, nx, ny, aux, counters);
+  ACK(cudaGetLastError());
+  int cnt[2] = {0, 0};
+  ACK(cudaMemcpyAsync(cnt, counters, sizeof(cnt), cudaMemcpyDeviceToHost, st));
+  ACK(cudaStreamSynchronize(st));
+  const long long n_irregular = cnt[0];
+  AdjScratch st_tab;
+  st_tab.add(&gat, (size_t)n_irregular * 3 * GMAX);
+  st_tab.add(&pul, (size_t)n_irregular * 3);
+  st_tab.add(&lkr, (size_t)n_irregular);
+  ACK(st_tab.alloc());
+  tables_kernel<<<grd, blk, 0, st>>>(L, h->d_mask, h->nxw, h->cfg.wall_y, aux, n_irregular, gat,
+                                     pul, lkr, counters);
+  count_launch(2);
+  ACK(cudaGetLastError());
+  ACK(cudaMemcpyAsync(cnt, counters, sizeof(cnt), cudaMemcpyDeviceToHost, st));
+  ACK(cudaStreamSynchronize(st));
+  if (cnt[1])
+    return afail(CFLBM_E_UNSUPPORTED, "cflbm_adjoint: more than 4 pulls read one population");
 
   // ---- forward run, keeping s_1, s_{K+1}, s_{2K+1}, ... ---------------------------
   const auto t_f0 = clk::now();
@@ -581,11 +740,7 @@ int run_adjoint(cflbm_handle *h, const cflbm_adjoint_spec *sp, double *dJ_dalpha
   // state s_T has lambda_{T+1} = 0) and the last (nothing left to recompute)
   // run as direct launches.
   const auto t_r0 = clk::now();
-  int *d_seg = nullptr;  // [0]: segment being reversed, [1]: segment being recomputed
-  double *c_tab = nullptr;
-  ACK(sc.alloc(&d_seg, 2));
-  ACK(sc.alloc(&c_tab, (size_t)T + 2));
-  {
+  {  // d_seg[0]: segment being reversed, [1]: segment being recomputed
     std::vector<double> ct((size_t)T + 2, 0.0);
     for (int t = t0; t <= t1; ++t) ct[t] = cw;
     const int k_last[2] = {nck - 1, nck - 1};
@@ -604,9 +759,15 @@ int run_adjoint(cflbm_handle *h, const cflbm_adjoint_spec *sp, double *dJ_dalpha
   aa.gat = gat;
   aa.pul = pul;
   aa.lkr = lkr;
+  aa.nirr = (int)n_irregular;
   aa.alpha = h->d_alpha;
   aa.omega = h->omega;
   aa.u_in = h->cfg.u0;
+  for (int j = 0; j < 9; ++j) {
+    aa.fin[j] = inlet_f(j, h->cfg.u0);
+    aa.fin_f[j] = (float)aa.fin[j];
+    aa.dfin[j] = inlet_dfdu(j, h->cfg.u0);
+  }
   aa.obj_axis = sp->objective;
   aa.g_alpha = ga;
   aa.g_block = gblk;
@@ -625,11 +786,7 @@ int run_adjoint(cflbm_handle *h, const cflbm_adjoint_spec *sp, double *dJ_dalpha
                                                         reinterpret_cast<uint4 *>(b));
     for (int q = 1; q < n; ++q) {
       SweepArgs sa = channel_args(h, b + (size_t)(q - 1) * sb, b + (size_t)q * sb, false);
-      sa.partials = scr_part;
-      sa.counter = scr_cnt;
-      sa.hist = scr_hist;
-      sa.step = scr_step;
-      sa.cap = 1;
+      sa.bnd_blocks = 0;  // the force of these steps is known
       ACK(launch_sweep_channel(9, h->cfg.storage, h->cfg.compute, sa, s));
     }
     step_back_kernel<<<1, 1, 0, s>>>(d_seg + 1);
@@ -639,13 +796,26 @@ int run_adjoint(cflbm_handle *h, const cflbm_adjoint_spec *sp, double *dJ_dalpha
   };
   // Reverse one segment of n states held in b (main stream).
   auto reverse = [&](char *b, int n, bool skip_top) -> int {
+    bool chained = false;
     for (int q = n - 1; q >= 0; --q) {
       if (skip_top && q == n - 1) continue;
       aa.s = b + (size_t)q * sb;
       aa.q = q;
       aa.mu_next = mu_next;
       aa.mu_out = mu_cur;
-      adjoint_kernel<A, false><<<grd, blk, 0, st>>>(aa);
+      // chained to the reverse step before it; the unit's first one also waits for
+      // the other stream and starts plainly
+      cudaLaunchAttribute at{};
+      at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at.val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t lc{};
+      lc.gridDim = grd;
+      lc.blockDim = blk;
+      lc.stream = st;
+      lc.attrs = &at;
+      lc.numAttrs = chained ? 1 : 0;
+      ACK(cudaLaunchKernelEx(&lc, adjoint_kernel<A, false>, aa));
+      chained = true;
       count_launch(1);
       std::swap(mu_next, mu_cur);
     }
@@ -684,7 +854,9 @@ int run_adjoint(cflbm_handle *h, const cflbm_adjoint_spec *sp, double *dJ_dalpha
   long long graph_launches = 0;
   for (int k = nck - 2; k >= 1; --k) {
     const int gi = (k & 1) * 2 + (mu_next == mu1 ? 0 : 1);
-    if (!gexec[gi]) {
+    if (nck - 2 < GRAPH_UNITS) {
+      if ((urc = unit(k, K, false))) return urc;
+    } else if (!gexec[gi]) {
       const long long n0 = cflbm_launch_count();
       cudaGraph_t g = nullptr;
       ACK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -718,7 +890,7 @@ int run_adjoint(cflbm_handle *h, const cflbm_adjoint_spec *sp, double *dJ_dalpha
   aa.seg = nullptr;
   aa.c_next = (1 >= t0 && 1 <= t1) ? cw : 0.0;
   adjoint_kernel<A, true><<<grd, blk, 0, st>>>(aa);
-  init_sens_kernel<A><<<grd, blk, 0, st>>>(aa, mu_cur, v0, ga64);
+  init_sens_kernel<A><<<grd, blk, 0, st>>>(aa, mu_cur, h->cfg.seed, h->cfg.perturb_amp, ga64);
   count_launch(2);
   ACK(cudaGetLastError());
   std::vector<double> hgb(2 * nblk);
@@ -738,7 +910,7 @@ int run_adjoint(cflbm_handle *h, const cflbm_adjoint_spec *sp, double *dJ_dalpha
   res->seconds_forward = t_forward;
   res->seconds_reverse = t_reverse;
   res->device_bytes = (int64_t)((size_t)(nck + 2 * K) * sb + (2 * 9 + 1) * N * sizeof(A) +
-                                N * (8 + 8 + 4) + n_irregular * (9 * GMAX * 8 + 9 * 8 + 4) +
+                                N * (8 + 4) + n_irregular * (3 * GMAX + 3 + 1) * 4 +
                                 2 * nblk * 8);
   return CFLBM_OK;
 }
