@@ -1,5 +1,6 @@
 // C ABI of the solver (include/cflbm.h): handle life cycle and the step loop.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -7,8 +8,10 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <exception>
 #include <thread>
 #include <vector>
+#include <unistd.h>
 #include <cuda.h>
 #include "handle.hpp"
 #include "setup.cuh"
@@ -68,7 +71,7 @@ void free_handle(cflbm_handle *h) {
                   h->d_face_off, h->d_face_bb, h->d_bcell_idx, h->d_bcell_links,
                   h->d_mw,  h->d_mp,   h->d_inlet, h->d_alpha, h->d_fin,    h->d_hist,
                   h->d_step, h->d_partials, h->d_counter, h->d_counter2, h->d_sums,
-                  h->d_err};
+                  h->d_err, h->d_stage};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
@@ -887,6 +890,69 @@ static int ensure_macros(cflbm_handle *h) {
   return CFLBM_OK;
 }
 
+extern "C++" {
+// Maps the pages of a host buffer that is about to be overwritten, on several cores
+// ahead of the copies into it.  A dump into fresh memory was bound by the driver's
+// page faults on one core: 226 MB took 7.8-9.9 ms, 1.2 ms once the pages are there;
+// mapped by 8 cores just ahead of 32 MB copies 2.1 ms (4 cores 2.4; MADV_POPULATE_WRITE
+// on 4 / 8 cores, which contend for the address space, 3.9 / 6.7; a pinned bounce
+// buffer emptied by 8 / 12 cores 4.0 / 3.7).
+class PageMapper {
+ public:
+  PageMapper(void *p, size_t bytes) : p_(static_cast<char *>(p)), bytes_(bytes) {
+    if (bytes < (8u << 20)) return;
+    try {
+      done_ = std::vector<std::atomic<char>>((bytes + PIECE - 1) / PIECE);
+      const unsigned n = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
+      pool_.reserve(n);
+      for (unsigned t = 0; t < n; ++t) pool_.emplace_back([this] { work(); });
+    } catch (const std::exception &) {  // no more threads or memory: with what there is
+    }
+  }
+  ~PageMapper() {
+    next_ = done_.size();
+    for (auto &t : pool_) t.join();
+  }
+  // Returns when the first `upto` bytes are mapped.
+  void wait(size_t upto) {
+    if (pool_.empty()) return;
+    for (; ready_ < done_.size() && ready_ * PIECE < upto; ++ready_)
+      while (!done_[ready_].load(std::memory_order_acquire)) std::this_thread::yield();
+  }
+
+ private:
+  static constexpr size_t PIECE = 2u << 20;
+  void work() {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    for (size_t k; (k = next_.fetch_add(1)) < done_.size();) {
+      const size_t e = std::min(bytes_, (k + 1) * PIECE);
+      for (size_t o = k * PIECE; o < e; o += page) static_cast<volatile char *>(p_)[o] = 0;
+      static_cast<volatile char *>(p_)[e - 1] = 0;
+      done_[k].store(1, std::memory_order_release);
+    }
+  }
+  char *p_;
+  size_t bytes_, ready_ = 0;
+  std::atomic<size_t> next_{0};
+  std::vector<std::atomic<char>> done_;
+  std::vector<std::thread> pool_;
+};
+
+// Device to host, into memory that may not be mapped yet.
+constexpr size_t STAGE_BYTES = 32u << 20;
+cudaError_t copy_out(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+  PageMapper map(dst, bytes);
+  cudaError_t e = cudaSuccess;
+  for (size_t o = 0; o < bytes && e == cudaSuccess; o += STAGE_BYTES) {
+    const size_t n = std::min(STAGE_BYTES, bytes - o);
+    map.wait(o + n);
+    e = cudaMemcpyAsync(static_cast<char *>(dst) + o, static_cast<const char *>(src) + o, n,
+                        cudaMemcpyDeviceToHost, s);
+  }
+  return e;
+}
+}  // extern "C++"
+
 int cflbm_macros(cflbm_handle *h, double *u, double *v, double *w, double *p) {
   if (!h) return fail(CFLBM_E_INVALID, "handle is NULL");
   CK_CUDA(cudaSetDevice(h->cfg.device));
@@ -895,7 +961,7 @@ int cflbm_macros(cflbm_handle *h, double *u, double *v, double *w, double *p) {
   double *dst[4] = {u, v, w, p};
   double *src[4] = {h->d_mu, h->d_mv, h->d_mw, h->d_mp};
   for (int k = 0; k < 4; ++k)
-    if (dst[k]) CK_CUDA(cudaMemcpyAsync(dst[k], src[k], N * 8, cudaMemcpyDeviceToHost, h->stream));
+    if (dst[k]) CK_CUDA(copy_out(dst[k], src[k], N * 8, h->stream));
   CK_CUDA(cudaStreamSynchronize(h->stream));
   return CFLBM_OK;
 }
@@ -1044,31 +1110,57 @@ int cflbm_mass(cflbm_handle *h, double *mass, double momentum[3]) {
   return CFLBM_OK;
 }
 
+// Dump / restore staging of a handle: device memory for a few MB of rows, kept (a
+// cudaMalloc and cudaFree of the whole dense state cost 0.3-0.5 ms per call).
+static int stage_rows(cflbm_handle *h, size_t row_bytes, size_t rows, size_t *per) {
+  const size_t want = std::max(row_bytes, std::min(STAGE_BYTES, row_bytes * rows));
+  if (h->stage_bytes < want) {
+    if (h->d_stage) {
+      CK_CUDA(cudaFree(h->d_stage));
+      h->device_bytes -= h->stage_bytes;
+      h->d_stage = nullptr;
+      h->stage_bytes = 0;
+    }
+    if (int rc = dev_alloc(h, reinterpret_cast<void **>(&h->d_stage), want)) return rc;
+    h->stage_bytes = want;
+  }
+  *per = std::max<size_t>(1, h->stage_bytes / row_bytes);
+  return CFLBM_OK;
+}
+
 int cflbm_get_f(cflbm_handle *h, double *out) {
   if (!h || !out) return fail(CFLBM_E_INVALID, "bad arguments");
   CK_CUDA(cudaSetDevice(h->cfg.device));
-  const size_t n = (size_t)h->Q * h->L.nx * h->L.ny * h->L.nz;
-  double *d = nullptr;
-  CK_CUDA(cudaMalloc(&d, n * sizeof(double)));
-  cudaError_t e = launch_get_f(h->Q, h->cfg.storage, h->L, h->fA, d, h->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(out, d, n * 8, cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  cudaFree(d);
-  CK_CUDA(e);
+  const size_t nx = h->L.nx, rows = (size_t)h->Q * h->L.ny * h->L.nz;
+  size_t per = 0;
+  if (int rc = stage_rows(h, nx * 8, rows, &per)) return rc;
+  PageMapper map(out, rows * nx * 8);
+  for (size_t r = 0; r < rows; r += per) {
+    const size_t n = std::min(per, rows - r);
+    CK_CUDA(launch_dense_rows(h->Q, h->cfg.storage, h->L, h->fA, h->d_stage, (long long)r,
+                              (long long)n, false, h->stream));
+    map.wait((r + n) * nx * 8);
+    CK_CUDA(cudaMemcpyAsync(out + r * nx, h->d_stage, n * nx * 8, cudaMemcpyDeviceToHost,
+                            h->stream));
+  }
+  CK_CUDA(cudaStreamSynchronize(h->stream));
   return CFLBM_OK;
 }
 
 int cflbm_set_f(cflbm_handle *h, const double *in, int64_t steps_done) {
   if (!h || !in || steps_done < 0) return fail(CFLBM_E_INVALID, "bad arguments");
   CK_CUDA(cudaSetDevice(h->cfg.device));
-  const size_t n = (size_t)h->Q * h->L.nx * h->L.ny * h->L.nz;
-  double *d = nullptr;
-  CK_CUDA(cudaMalloc(&d, n * sizeof(double)));
-  cudaError_t e = cudaMemcpyAsync(d, in, n * 8, cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess) e = launch_set_f(h->Q, h->cfg.storage, h->L, h->fA, d, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  cudaFree(d);
-  CK_CUDA(e);
+  const size_t nx = h->L.nx, rows = (size_t)h->Q * h->L.ny * h->L.nz;
+  size_t per = 0;
+  if (int rc = stage_rows(h, nx * 8, rows, &per)) return rc;
+  for (size_t r = 0; r < rows; r += per) {
+    const size_t n = std::min(per, rows - r);
+    CK_CUDA(cudaMemcpyAsync(h->d_stage, in + r * nx, n * nx * 8, cudaMemcpyHostToDevice,
+                            h->stream));
+    CK_CUDA(launch_dense_rows(h->Q, h->cfg.storage, h->L, h->fA, h->d_stage, (long long)r,
+                              (long long)n, true, h->stream));
+  }
+  CK_CUDA(cudaStreamSynchronize(h->stream));
   h->steps_done = steps_done;
   // fields handed out directly can still be formed from fB
   h->macros_pending = h->macros_pending && h->macros_direct;
@@ -1089,7 +1181,7 @@ int cflbm_get_f_stream(cflbm_handle *h, double *out) {
   SweepArgs sa = channel_args(h, h->fB, nullptr, false);
   cudaError_t e = launch_stream_state(h->Q, h->cfg.storage, sa,
                                       h->cfg.profile != CFLBM_PROFILE_CHANNEL, d, h->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(out, d, n * 8, cudaMemcpyDeviceToHost, h->stream);
+  if (e == cudaSuccess) e = copy_out(out, d, n * 8, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   cudaFree(d);
   CK_CUDA(e);

@@ -52,6 +52,8 @@ struct cflbm_handle {
   unsigned int *d_counter = nullptr;   // links kernel
   unsigned int *d_counter2 = nullptr;  // mass kernel
   double *d_sums = nullptr;            // 4 doubles (mass, momentum)
+  double *d_stage = nullptr;           // dump / restore staging, made on first use
+  size_t stage_bytes = 0;
   unsigned *d_err = nullptr;           // device error word (a bounded wait gave up)
   bool lines = false;                  // the interior runs the line-staged sweep
   long long steps_done = 0;

@@ -190,10 +190,9 @@ cudaError_t launch_init_channel(int Q, int store, const Layout &L, void *f,
                                 double *mu, double *mv, double *mw, double *mp, cudaStream_t s);
 cudaError_t launch_reduce_mass(int Q, int store, const ReduceArgs &a, int blocks,
                                cudaStream_t s);
-cudaError_t launch_get_f(int Q, int store, const Layout &L, const void *f, double *out,
-                         cudaStream_t s);
-cudaError_t launch_set_f(int Q, int store, const Layout &L, void *f, const double *in,
-                         cudaStream_t s);
+// Rows [r0, r0 + n) of the dense [i][z][y][x] state to (or, put, from) `dense`.
+cudaError_t launch_dense_rows(int Q, int store, const Layout &L, void *f, double *dense,
+                              long long r0, long long n, bool put, cudaStream_t s);
 cudaError_t launch_fill_value(int Q, int store, const Layout &L, void *f, cudaStream_t s);
 
 // Fill omega, omega_f and the relaxation constants rk/rkf and fx of a sweep for
