@@ -356,6 +356,13 @@ int cflbm_create(const cflbm_config *cfg, cflbm_handle **out) {
     else build_links<9>(solid, nx, ny, nz, links, h->n_solid);
     h->n_links = (long long)links.size();
     mask = pack_mask(solid, nx, ny, nz, h->nxw);
+    // no solid cell within two cells of a face (see ref_boundary_kernel)
+    h->links_inside = true;
+    for (const int4 &l : links) {
+      const int c[3] = {l.x, l.y, l.z}, n[3] = {nx, ny, nz};
+      for (int d = 0; d < (d3 ? 3 : 2); ++d)
+        if (c[d] < 2 || c[d] > n[d] - 3) h->links_inside = false;
+    }
   }
 
   // Device allocations.
@@ -474,7 +481,8 @@ int cflbm_create(const cflbm_config *cfg, cflbm_handle **out) {
     }
     CK_CUDA(cudaStreamSynchronize(h->stream));  // host vectors die at scope end
   }
-  h->link_blocks = (int)std::min<long long>(std::max<long long>((h->n_links + 255) / 256, 1), 1024);
+  // up to 4 links per thread in one block: its sum needs no partials
+  h->link_blocks = h->n_links <= 1024 ? 1 : (int)std::min<long long>((h->n_links + 255) / 256, 1024);
   // Force partials: one per block of listed tiles, for any tile height >= 1.
   const size_t nparts = std::max<size_t>(4 * (size_t)std::max(h->link_blocks, h->reduce_blocks),
                                          3 * (size_t)std::max(h->n_slow, 1));
@@ -527,7 +535,7 @@ int cflbm_create(const cflbm_config *cfg, cflbm_handle **out) {
     cudaMemcpyAsync(dp, ref.p.data(), P * 8, cudaMemcpyHostToDevice, h->stream);
     cudaError_t e = launch_init_macros(Q, cfg->storage, L, h->fA, du, dv, dw, dp, h->stream);
     // Both buffers start with the same ghost layers; afterwards only the face
-    // passes write ghosts, into both buffers.
+    // passes write ghosts, into the buffer of their step.
     if (e == cudaSuccess) e = launch_ghost_copy(Q, cfg->storage, L, h->fA, h->fB, h->stream);
     // Step-0 macroscopic fields: the interior of the initial fields.
     std::vector<double> mu(N), mv(N), mw(N), mp(N);
@@ -725,7 +733,7 @@ static int one_step(cflbm_handle *h, bool write_macros) {
   FillArgs fa{};
   fa.L = L;
   fa.f = h->fA;
-  fa.f2 = h->fB;  // face-pass ghosts go to both buffers (see face_op_kernel)
+  fa.f2 = h->fB;
   fa.mask = h->d_mask;
   fa.nxw = h->nxw;
   fa.wall_y = h->cfg.wall_y;
@@ -748,34 +756,35 @@ static int one_step(cflbm_handle *h, bool write_macros) {
     h->macros_direct = false;
     return CFLBM_OK;
   }
-  if (h->cfg.profile == CFLBM_PROFILE_REF2D || h->cfg.profile == CFLBM_PROFILE_REF2DS) {
-    // "MPI Kokkos/lbm.cpp:315-345": inlet, outlet, then the two wall rows.
-    // Each pair (the two ends of one axis) writes and reads disjoint layers, so a
-    // pair runs as one launch; the pairs keep the reference's order.  The serial
-    // variant's wall rows ("Kokkos/lbm.cpp:158-168") leave out the two corner
-    // nodes of each ghost row.
-    const int trim = h->cfg.profile == CFLBM_PROFILE_REF2DS ? 1 : 0;
-    const FaceOp ops[4] = {{0, 0, 0, 0}, {1, 0, 1, 0}, {2, 1, 0, trim}, {2, 1, 1, trim}};
-    for (int k = 0; k < 4; k += 2)
-      CK_CUDA(launch_face_ops(Q, st, fa, ops[k], ops[k + 1], h->stream));
-  } else {
-    // "3D MPI+KOKKOS+MPIIO/lbm.cpp:278-347": front, back, bottom, top, inlet, outlet.
-    const FaceOp ops[6] = {{2, 1, 0}, {2, 1, 1}, {2, 2, 0}, {2, 2, 1}, {0, 0, 0}, {1, 0, 1}};
-    for (int k = 0; k < 6; k += 2)
-      CK_CUDA(launch_face_ops(Q, st, fa, ops[k], ops[k + 1], h->stream));
-  }
   LinkArgs la{};
   la.L = L;
   la.f = h->fA;
   la.links = h->d_links;
   la.n = h->n_links;
-  la.reach = ref ? 2 : 1;
+  la.reach = 2;
+  la.blocks = h->link_blocks;
   la.partials = h->d_partials;
   la.counter = h->d_counter;
   la.hist = h->d_hist;
   la.step = h->d_step;
   la.cap = h->hist_cap;
-  CK_CUDA(launch_links(Q, st, la, h->link_blocks, h->stream));
+  // "MPI Kokkos/lbm.cpp:315-345": inlet, outlet, then the two wall rows.  The serial
+  // variant's wall rows ("Kokkos/lbm.cpp:158-168") leave out the two corner nodes of
+  // each ghost row.  "3D MPI+KOKKOS+MPIIO/lbm.cpp:278-347": front, back, bottom, top,
+  // inlet, outlet.
+  const int trim = h->cfg.profile == CFLBM_PROFILE_REF2DS ? 1 : 0;
+  const FaceOp ops2[4] = {{0, 0, 0, 0}, {1, 0, 1, 0}, {2, 1, 0, trim}, {2, 1, 1, trim}};
+  const FaceOp ops3[6] = {{2, 1, 0}, {2, 1, 1}, {2, 2, 0}, {2, 2, 1}, {0, 0, 0}, {1, 0, 1}};
+  const FaceOp *ops = Q == 9 ? ops2 : ops3;
+  const int nops = Q == 9 ? 4 : 6;
+  if (h->links_inside) {
+    CK_CUDA(launch_ref_boundary(Q, st, fa, ops, nops, la, h->stream));
+  } else {
+    LinkArgs none = la;
+    none.blocks = 0;
+    CK_CUDA(launch_ref_boundary(Q, st, fa, ops, nops, none, h->stream));
+    CK_CUDA(launch_ref_boundary(Q, st, fa, ops, 0, la, h->stream));
+  }
   if (h->timing) {
     if ((trc = record_event(h, &tb1))) return trc;
     h->bnd_ev.push_back({tb0, tb1});

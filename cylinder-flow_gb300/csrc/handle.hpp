@@ -48,6 +48,7 @@ struct cflbm_handle {
   long long *d_step = nullptr;
   double *d_partials = nullptr;
   int link_blocks = 1;
+  bool links_inside = false;  // reference profiles: links and face passes are independent
   int reduce_blocks = 1;
   unsigned int *d_counter = nullptr;   // links kernel
   unsigned int *d_counter2 = nullptr;  // mass kernel

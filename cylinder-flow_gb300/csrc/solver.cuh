@@ -121,7 +121,7 @@ struct SweepArgs {
 struct FillArgs {
   Layout L;
   void *f;               // state being filled (in place)
-  void *f2;              // the other buffer: face passes write their ghosts here too (or null)
+  const void *f2;        // the other buffer: the ghosts of the step before
   const uint32_t *mask;
   int nxw;
   int wall_y, wall_z;
@@ -133,8 +133,15 @@ struct FaceOp {
   int axis;  // 0 x, 1 y, 2 z
   int side;  // 0 low, 1 high
   int trim;  // 1: the pass skips the two ghost ends of its tangential range
-  int ndir;  // the populations the pass writes (filled by launch_face_ops),
+  int ndir;  // the populations the pass writes (filled by launch_ref_boundary),
   unsigned long long dirs;  // 5 bits each, the k-th at bit 5k
+};
+
+// The passes of a step in their order; start: first thread of each.
+struct FaceOps {
+  int n;
+  int start[7];
+  FaceOp op[6];
 };
 
 struct LinkArgs {
@@ -143,6 +150,7 @@ struct LinkArgs {
   const int4 *links;     // (x, y, z, k): solid cell s, direction k, s + e_k fluid
   long long n;
   int reach;             // 1: halfway bounce-back, 2: the reference's s + 2 e_k rule
+  int blocks;            // blocks of the launch that do links (0: none)
   double *partials;      // 3 doubles per block
   unsigned int *counter; // last-block detection, self-resetting
   double *hist;          // force history, 3 doubles per slot
@@ -175,12 +183,12 @@ cudaError_t launch_stream_state(int Q, int store, const SweepArgs &a, bool ref, 
 // (the solid-tile launch runs 4 listed warp tiles per block).
 constexpr int SWEEP_BX = 32, SWEEP_BY = 4;
 cudaError_t launch_fill_channel(int Q, int store, const FillArgs &a, cudaStream_t s);
-// Two face passes of one axis (independent of each other) in one launch.
-cudaError_t launch_face_ops(int Q, int store, const FillArgs &a, FaceOp op0, FaceOp op1,
-                            cudaStream_t s);
+// The face passes op[0..nops) of a step and, with la.blocks > 0, its link fill, as one
+// launch (both only where neither reads what the other writes).
+cudaError_t launch_ref_boundary(int Q, int store, const FillArgs &a, const FaceOp *op, int nops,
+                                const LinkArgs &la, cudaStream_t s);
 cudaError_t launch_ghost_copy(int Q, int store, const Layout &L, const void *src, void *dst,
                               cudaStream_t s);
-cudaError_t launch_links(int Q, int store, const LinkArgs &a, int blocks, cudaStream_t s);
 cudaError_t launch_init_macros(int Q, int store, const Layout &L, void *f, const double *u,
                                const double *v, const double *w, const double *p,
                                cudaStream_t s);

@@ -306,6 +306,12 @@ __device__ __forceinline__ void finish_cell(A *f, A rho3, A ux, A uy, A uz, long
   }
 }
 
+// Programmatic dependent launch (the steps): a kernel starts while its
+// predecessor on the stream runs; wait() returns when that has finished and its
+// writes are visible.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- reference profiles --------------------------------------------------------
 template <int Q, class ST, class A, int MINB>
 __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_kernel(const SweepArgs a) {
@@ -321,14 +327,16 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_kernel(const 
   const E *__restrict__ fa = static_cast<const E *>(a.fa);
   E *__restrict__ fb = static_cast<E *>(a.fb);
 
+  const bool solid = mask_solid(a.mask, a.nxw, a.L.ny, x, y, z);
+  pdl_wait();
   A f[Q];
 #pragma unroll
   for (int i = 0; i < Q; ++i)
     f[i] = SF::template load<A, L>(fa + i * S + c - a.L.off(L::ex(i), L::ey(i), L::ez(i)),
                                    a.L.fbase[i]);
+  pdl_trigger();
 
   const long long cell = ((long long)z * a.L.ny + y) * a.L.nx + x;
-  const bool solid = mask_solid(a.mask, a.nxw, a.L.ny, x, y, z);
   if constexpr (std::is_same<A, double>::value) {
     const bool in = a.ref_override && x == 0;
     if (fixed_cell<L, SF>(f, solid, in, in ? a.inlet_u[(long long)z * a.L.ny + y] : 0.0,
@@ -355,9 +363,18 @@ template <int Q, class ST, class A, int MINB>
 cudaError_t launch_sweep_t(const SweepArgs &a, cudaStream_t s) {
   dim3 block(SWEEP_BX, SWEEP_BY, 1);
   dim3 grid((a.L.nx + SWEEP_BX - 1) / SWEEP_BX, (a.L.ny + SWEEP_BY - 1) / SWEEP_BY, a.L.nz);
-  sweep_kernel<Q, ST, A, MINB><<<grid, block, 0, s>>>(a);
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, sweep_kernel<Q, ST, A, MINB>, a);
   count_launch();
-  return cudaGetLastError();
+  return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 // ---- channel profile -------------------------------------------------------------
@@ -757,12 +774,6 @@ __device__ __forceinline__ void channel2_cells(const SweepArgs &a, int x0, int y
     PairCodec<ST>::template put2<Q>(q + i * S, q + i * S + 32, f[i], a.L.fbase[i], st0, st1,
                                     (unsigned)(cell0 * Q + i), a.f16_sr);
 }
-
-// Programmatic dependent launch (the one-launch step): a kernel starts while its
-// predecessor on the stream runs; wait() returns when that has finished and its
-// writes are visible.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Sums per-thread FP64 force partials over `nblk` blocks, this one number `blk`:
 // warp shuffles, per block, and over blocks, in block order, by the last block to
