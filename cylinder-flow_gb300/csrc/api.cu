@@ -79,6 +79,7 @@ void free_handle(cflbm_handle *h) {
     if (g) cudaGraphExecDestroy(g);
   if (h->ev_sync) cudaEventDestroy(h->ev_sync);
   if (h->stream) cudaStreamDestroy(h->stream);
+  if (h->force_host) cudaFreeHost(const_cast<double *>(h->force_host));
   delete h;
 }
 
@@ -242,6 +243,10 @@ int validate(const cflbm_config *c) {
 }
 
 }  // namespace
+
+namespace cflbm {
+static void init_args(cflbm_handle *h);
+}
 
 extern "C" {
 
@@ -559,6 +564,7 @@ int cflbm_create(const cflbm_config *cfg, cflbm_handle **out) {
     CK_CUDA(e);
     CK_CUDA(e2);
   }
+  init_args(h);
   CK_CUDA(cudaStreamSynchronize(h->stream));
   CK_CUDA(cudaGetLastError());
   *out = hp.release();
@@ -670,23 +676,24 @@ void set_offsets(SweepArgs &a, int Q) {
   }
 }
 
-// Arguments of the channel sweep of handle h reading fa and writing fb.
-SweepArgs channel_args(const cflbm_handle *h, const void *fa, void *fb, bool write_macros) {
-  SweepArgs sa{};
+// The arguments that every sweep of a handle shares, formed once (their constants
+// cost the host about as much as a launch).
+static void init_args(cflbm_handle *h) {
+  SweepArgs &sa = h->args;
+  sa = SweepArgs{};
   sa.L = h->L;
-  sa.fa = fa;
-  sa.fb = fb;
   sa.mask = h->d_mask;
   sa.nxw = h->nxw;
   set_relax(sa, h->Q, h->cfg.storage, h->omega);
   set_offsets(sa, h->Q);
   sa.f16_sr = h->cfg.rounding == CFLBM_ROUND_STOCHASTIC;
   sa.alpha = h->d_alpha;
-  if (write_macros) {
-    sa.mu = h->d_mu;
-    sa.mv = h->d_mv;
-    sa.mw = h->d_mw;
-    sa.mp = h->d_mp;
+  sa.sms = h->sms;
+  sa.err = h->d_err;
+  if (h->cfg.profile != CFLBM_PROFILE_CHANNEL) {
+    sa.ref_override = 1;
+    sa.inlet_u = h->d_inlet;
+    return;
   }
   sa.wall_y = h->cfg.wall_y;
   sa.wall_z = h->cfg.wall_z;
@@ -714,15 +721,26 @@ SweepArgs channel_args(const cflbm_handle *h, const void *fa, void *fb, bool wri
   sa.hist = h->d_hist;
   sa.step = h->d_step;
   sa.cap = h->hist_cap;
-  sa.sms = h->sms;
   sa.lines = h->lines ? 1 : 0;
-  sa.err = h->d_err;
+}
+
+// Arguments of the sweep of handle h reading fa and writing fb.
+SweepArgs channel_args(const cflbm_handle *h, const void *fa, void *fb, bool write_macros) {
+  SweepArgs sa = h->args;
+  sa.fa = fa;
+  sa.fb = fb;
+  if (write_macros) {
+    sa.mu = h->d_mu;
+    sa.mv = h->d_mv;
+    sa.mw = h->d_mw;
+    sa.mp = h->d_mp;
+  }
   return sa;
 }
 }  // namespace cflbm
 }  // extern "C++"
 
-static int one_step(cflbm_handle *h, bool write_macros) {
+static int one_step(cflbm_handle *h, bool last) {
   size_t tb0 = 0, tb1 = 0, ts0 = 0, ts1 = 0;
   int trc;
   if (h->timing && h->cfg.profile != CFLBM_PROFILE_CHANNEL && (trc = record_event(h, &tb0)))
@@ -730,20 +748,11 @@ static int one_step(cflbm_handle *h, bool write_macros) {
   const int Q = h->Q;
   const int st = h->cfg.storage;
   const Layout &L = h->L;
-  FillArgs fa{};
-  fa.L = L;
-  fa.f = h->fA;
-  fa.f2 = h->fB;
-  fa.mask = h->d_mask;
-  fa.nxw = h->nxw;
-  fa.wall_y = h->cfg.wall_y;
-  fa.wall_z = h->cfg.wall_z;
-  fa.f_in = h->d_fin;
-  const bool ref = h->cfg.profile != CFLBM_PROFILE_CHANNEL;
-  if (!ref) {
-    // u, v, w, p are formed on request (ensure_macros), not written every step.
-    (void)write_macros;
-    const SweepArgs sa = channel_args(h, h->fA, h->fB, false);
+  if (h->cfg.profile == CFLBM_PROFILE_CHANNEL) {
+    // u, v, w, p are formed on request (ensure_macros), not written every step;
+    // `last`: the force also goes where cflbm_forces reads it.
+    SweepArgs sa = channel_args(h, h->fA, h->fB, false);
+    if (last) sa.force_host = h->d_force_host;
     if (h->timing && (trc = record_event(h, &ts0))) return trc;
     CK_CUDA(launch_sweep_channel(Q, st, h->cfg.compute, sa, h->stream));
     if (h->timing) {
@@ -752,10 +761,15 @@ static int one_step(cflbm_handle *h, bool write_macros) {
     }
     std::swap(h->fA, h->fB);
     ++h->steps_done;
+    if (last && h->d_force_host) h->force_host_step = h->steps_done;
     h->macros_pending = true;
     h->macros_direct = false;
     return CFLBM_OK;
   }
+  FillArgs fa{};
+  fa.L = L;
+  fa.f = h->fA;
+  fa.f2 = h->fB;
   LinkArgs la{};
   la.L = L;
   la.f = h->fA;
@@ -790,24 +804,7 @@ static int one_step(cflbm_handle *h, bool write_macros) {
     h->bnd_ev.push_back({tb0, tb1});
     if ((trc = record_event(h, &ts0))) return trc;
   }
-  SweepArgs sa{};
-  sa.L = L;
-  sa.fa = h->fA;
-  sa.fb = h->fB;
-  sa.mask = h->d_mask;
-  sa.nxw = h->nxw;
-  set_relax(sa, Q, st, h->omega);
-  set_offsets(sa, Q);
-  sa.f16_sr = h->cfg.rounding == CFLBM_ROUND_STOCHASTIC;
-  sa.ref_override = ref ? 1 : 0;
-  sa.inlet_u = h->d_inlet;
-  sa.alpha = h->d_alpha;
-  if (write_macros) {
-    sa.mu = h->d_mu;
-    sa.mv = h->d_mv;
-    sa.mw = h->d_mw;
-    sa.mp = h->d_mp;
-  }
+  const SweepArgs sa = channel_args(h, h->fA, h->fB, last);
   CK_CUDA(launch_sweep(Q, st, h->cfg.compute, sa, h->stream));
   if (h->timing) {
     if ((trc = record_event(h, &ts1))) return trc;
@@ -1035,12 +1032,28 @@ int cflbm_forces(cflbm_handle *h, double fxyz[3], double cd_cl[2]) {
   if (!h) return fail(CFLBM_E_INVALID, "handle is NULL");
   CK_CUDA(cudaSetDevice(h->cfg.device));
   double F[3] = {0.0, 0.0, 0.0};
-  if (h->steps_done > 0) {
+  if (h->force_host_step == h->steps_done && h->steps_done > 0) {
+    // the last step's kernel wrote it to pinned host memory: no copy to wait for
+    CK_CUDA(cudaStreamSynchronize(h->stream));
+    for (int d = 0; d < 3; ++d) F[d] = h->force_host[d];
+  } else if (h->steps_done > 0) {
+    if (!h->force_host && !h->batched && h->cfg.profile == CFLBM_PROFILE_CHANNEL) {
+      // a caller that asks for forces: from the next step on through pinned memory
+      // (without it the copy below, through pageable memory, goes on serving)
+      void *p = nullptr;
+      if (cudaHostAlloc(&p, 64, cudaHostAllocMapped) == cudaSuccess) {
+        h->force_host = static_cast<volatile double *>(p);
+        void *d = nullptr;
+        if (cudaHostGetDevicePointer(&d, p, 0) == cudaSuccess)
+          h->d_force_host = static_cast<double *>(d);
+      }
+      cudaGetLastError();
+    }
     const long long slot = (h->steps_done - 1) % h->hist_cap;
     CK_CUDA(cudaMemcpyAsync(F, h->d_hist + 3 * slot, 3 * sizeof(double), cudaMemcpyDeviceToHost,
                             h->stream));
   }
-  CK_CUDA(cudaStreamSynchronize(h->stream));
+  if (h->force_host_step != h->steps_done) CK_CUDA(cudaStreamSynchronize(h->stream));
   if (fxyz) {
     fxyz[0] = F[0];
     fxyz[1] = F[1];
@@ -1171,6 +1184,7 @@ int cflbm_set_f(cflbm_handle *h, const double *in, int64_t steps_done) {
   }
   CK_CUDA(cudaStreamSynchronize(h->stream));
   h->steps_done = steps_done;
+  h->force_host_step = -1;
   // fields handed out directly can still be formed from fB
   h->macros_pending = h->macros_pending && h->macros_direct;
   long long st = steps_done;

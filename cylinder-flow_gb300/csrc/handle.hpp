@@ -57,6 +57,12 @@ struct cflbm_handle {
   size_t stage_bytes = 0;
   unsigned *d_err = nullptr;           // device error word (a bounded wait gave up)
   bool lines = false;                  // the interior runs the line-staged sweep
+  // The force of the last step of a call, written by its kernel into pinned host
+  // memory once cflbm_forces has been called; the step it belongs to.
+  volatile double *force_host = nullptr;
+  double *d_force_host = nullptr;
+  long long force_host_step = -1;
+  cflbm::SweepArgs args;  // what every sweep of the handle shares (init_args)
   long long steps_done = 0;
   double omega = 1.0;
   double area = 1.0;  // Cd/Cl reference area

@@ -111,6 +111,7 @@ struct SweepArgs {
   double *hist;          // force history, 3 doubles per step
   long long *step;       // device step counter (history slot = step % cap)
   long long cap;
+  double *force_host;    // the force also here (pinned host memory) or null
   int bnd_blocks;        // blocks of the force (at most one per SM; 0: not formed)
   int force_span;        // leading grid rows (2-D) or planes (3-D) of the sweep that form it
   int sms;               // multiprocessors of the device

@@ -810,6 +810,11 @@ __device__ __forceinline__ void force_to_history(const SweepArgs &a, double dx, 
     h[1] = dy;
     h[2] = dz;
     *a.step = st + 1;
+    if (a.force_host) {
+      a.force_host[0] = dx;
+      a.force_host[1] = dy;
+      a.force_host[2] = dz;
+    }
   };
   block_sum(dx, dy, dz);
   if (nblk == 1) {
