@@ -34,15 +34,14 @@ namespace cflbm {
 constexpr int FX_P = 55;             // q_i = g_i 2^(FX_P - E)
 constexpr int FX_EMAX = 1023 - 3;    // largest biased exponent covered
 constexpr int FX_EMIN = 1023 - 900;  // smaller ones are raised to it
-// Populations 0 .. FX_NINT - 1 are converted to FP64 with integer operations, the
+// Populations 0 .. fx_nint - 1 are converted to FP64 with integer operations, the
 // others by the FP64 pipe: with all 54 conversions of a D3Q27 cell on it that pipe
 // binds (27 clocks per cell and SM), with all 27 outgoing ones off it the integer
-// pipes do.  10 steps and the fields of the 512x128x128 cylinder, ms: 9.34 / 8.86
-// / 8.54 / 8.46 / 8.39 / 8.48 / 8.70 for 0 / 6 / 10 / 14 / 18 / 22 / 27 (FP64
-// operations: 22.78); REF3D 257x97x97, 20 steps: 6.43 / 6.02 / 5.80 / 5.65 / 5.51
-// / 5.43 / 5.58 (15.17); D2Q9 400x100, 400 steps: 2.78 ms for none, 2.70 for all 9
-// (3.11).
-template <class L> constexpr int fx_nint = L::D == 3 ? 18 : 4;
+// pipes do.  10 steps and the fields of the 512x128x128 cylinder, ms: 7.50 / 7.40 /
+// 7.33 / 7.36 / 7.39 for 18 / 20 / 22 / 25 / 27 (with a longer conversion 9.34 for
+// none, 8.39 for 18; FP64 operations: 22.78); D2Q9 1132x168, 400 steps: 3.31 / 3.24 /
+// 3.22 / 3.25 for 3 / 4 / 5 / 6 (FP64 operations: 4.01).
+template <class L> constexpr int fx_nint = L::D == 3 ? 22 : 5;
 
 // Shift of the weight of class c = |e|^2 (w = W 2^k), the scale of the velocity
 // sums (u = M 2^(E - FX_P - FX_U)) and of rho3 (FX_R).
@@ -60,12 +59,17 @@ __device__ __forceinline__ Limbs limbs(long long x) {
   const unsigned lo = (unsigned)x;
   return {(int)(x >> 32) + (int)(lo >> 31), (int)lo};
 }
-// x c / 2^64 + add, rounded to nearest but for the product of the low limbs
-// (below a quarter of a unit, of either sign).
-__device__ __forceinline__ long long mul_hi(Limbs x, FxConst c, long long add) {
-  long long cross = (long long)x.l * c.h + 0x80000000LL;
+// x c / 2^64 + add + 2^31, rounded to nearest but for the product of the low limbs
+// (below a quarter of a unit, of either sign).  The cross terms carry 2^63 so that
+// their upper word needs no sign extension; callers take the FX_BIAS off once.
+constexpr long long FX_BIAS = 1LL << 31;
+__device__ __forceinline__ long long mul_hi_b(Limbs x, FxConst c, long long add) {
+  long long cross = (long long)x.l * c.h + (long long)0x8000000080000000ULL;
   cross = (long long)x.h * c.l + cross;
-  return (long long)x.h * c.h + ((cross >> 32) + add);
+  return (long long)x.h * c.h + (add + (long long)((unsigned long long)cross >> 32));
+}
+__device__ __forceinline__ long long mul_hi(Limbs x, FxConst c, long long add) {
+  return mul_hi_b(x, c, add - FX_BIAS);
 }
 __device__ __forceinline__ long long mul_hi(long long x, FxConst c, long long add = 0) {
   return mul_hi(limbs(x), c, add);
@@ -74,12 +78,15 @@ __device__ __forceinline__ long long mul_hi(Limbs x, Limbs y, long long add) {
   return mul_hi(x, FxConst{y.h, y.l}, add);
 }
 
-// Larger magnitude of two doubles' high words, as floats: the order of
+// Larger of m and the magnitudes of two doubles' high words, as floats: the order of
 // magnitudes is the words' order, and a word that is a float NaN (|d| >= 2^1017,
 // infinities and NaNs among them) wins.
-__device__ __forceinline__ float max_mag(float m, double d) {
+__device__ __forceinline__ float max_mag(float m, double d, double e) {
   float r;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(m), "f"(fabsf(__int_as_float(__double2hiint(d)))));
+  asm("max.NaN.f32 %0, %1, %2, %3;"
+      : "=f"(r)
+      : "f"(m), "f"(fabsf(__int_as_float(__double2hiint(d)))),
+        "f"(fabsf(__int_as_float(__double2hiint(e)))));
   return r;
 }
 
@@ -89,11 +96,12 @@ template <class L>
 __device__ __forceinline__ int fx_exponent(const double *f, double ux) {
   float m[L::D + 1] = {};
   static_for(
-      [&](auto ic) {
-        constexpr int I = decltype(ic)::value;
-        m[wclass<L>(I)] = max_mag(m[wclass<L>(I)], f[I]);
+      [&](auto kc) {
+        constexpr int i = L::pair(decltype(kc)::value), c = wclass<L>(i);
+        m[c] = max_mag(m[c], f[i], f[L::opp(i)]);
       },
-      std::make_integer_sequence<int, L::Q>{});
+      std::make_integer_sequence<int, L::NPAIR>{});
+  m[0] = max_mag(0.0f, f[0], f[0]);
   // |ux| <= 8 max |g| keeps its integer below 2^62
   int hi = (__double2hiint(ux) & 0x7FFFFFFF) - (3 << 20);
 #pragma unroll
@@ -107,16 +115,23 @@ __device__ __forceinline__ double scale_bits(double d, int s20) {
 }
 
 // x 2^(s20 / 2^20 - 1023) in FP64 (s20: the biased exponent of 1 in x's units, at
-// bit 20), rounded to nearest, on the integer pipes: 17 operations for the
-// conversion's slot of the FP64 pipe.
+// bit 20; |x| < 2^62), rounded to nearest, on the integer pipes.
 __device__ __forceinline__ double fx_to_double(long long x, int s20) {
-  const long long sg = x >> 63;
-  unsigned long long u = (unsigned long long)((x ^ sg) - sg);
-  const int z = __clzll((long long)u);
-  u = z < 64 ? u << z : 0;
-  const unsigned long long m = (u >> 11) + ((u >> 10) & 1);
-  const unsigned long long r = m + ((unsigned long long)(unsigned)(s20 + ((62 - z) << 20)) << 32);
-  return __longlong_as_double(u == 0 ? 0 : (long long)(r | ((unsigned long long)sg << 63)));
+  unsigned lo = (unsigned)x;
+  const unsigned sign = (unsigned)(x >> 32);
+  unsigned hi = sign;
+  asm("{\n\t.reg .pred p;\n\t"
+      "setp.lt.s32 p, %1, 0;\n\t"
+      "@p sub.cc.u32 %0, 0, %0;\n\t"
+      "@p subc.u32 %1, 0, %1;\n\t}"
+      : "+r"(lo), "+r"(hi));
+  const bool low = hi == 0u;
+  const int z = __clz((int)(low ? lo : hi)) + (low ? 31 : -1);  // to bit 62; 63 for zero
+  unsigned long long u = (((unsigned long long)hi << 32) | lo) << z;
+  u = (u + 0x200u) >> 10;  // 53 bits, the first one included; a carry enters the exponent
+  const int e = z == 63 ? 0 : s20 + ((61 - z) << 20);
+  return __hiloint2double((int)(((unsigned)(u >> 32) + (unsigned)e) | (sign & 0x80000000u)),
+                          (int)(unsigned)u);
 }
 
 // The populations as integers q_i and their moments: the cascade of moments_get
@@ -181,19 +196,19 @@ __device__ __forceinline__ void fx_store_macros(const SweepArgs &a, long long ce
   if (a.mp) a.mp[cell] = __ddiv_rn(__dmul_rn(__ll2double_rn(mr), sr), 3.0);
 }
 
-// Collision and store of one cell with FP64 arithmetic.  f: the pulled
-// populations.  solid: p = u = 0; inlet: u = (ux_in, 0, 0); outlet: p = 0 (the
+// Collision and store of one cell with FP64 arithmetic, population i to
+// fb[doff_i + at] (fb: the block's first cell).  f: the pulled populations.  solid: p = u = 0; inlet: u = (ux_in, 0, 0); outlet: p = 0 (the
 // reference profiles' rules).  Returns false, with nothing written, where the
 // format does not cover the cell.
 template <class L, class SF, class E>
 __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inlet, double ux_in,
                                            bool outlet, long long cell, bool store,
-                                           E *__restrict__ fb, long long c, long long S,
+                                           E *__restrict__ fb, unsigned at,
                                            const SweepArgs &a) {
   constexpr int D = L::D;
   const int eb = fx_exponent<L>(f, inlet && !solid ? ux_in : 0.0);
   double s = 1.0;
-  if (a.alpha) s = __dsub_rn(1.0, (double)a.alpha[cell]);
+  if (a.alpha && store) s = __dsub_rn(1.0, (double)a.alpha[cell]);
   if (!a.fx_ok || eb > FX_EMAX || !(fabs(s) <= 1.0)) return false;
 
   long long q[L::Q], mr, mu[3];
@@ -234,12 +249,13 @@ __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inl
   }
   long long qs = qd[0] + qd[1];
   if constexpr (D == 3) qs += qd[2];
-  const long long G = mul_hi(mr, a.fx[FX_G], -mul_hi(qs, a.fx[FX_THIRD]));
+  // less the bias that every population's product adds (mul_hi_b)
+  const long long G = mul_hi(mr, a.fx[FX_G], -mul_hi(qs, a.fx[FX_THIRD])) - FX_BIAS;
 
   const int out20 = (eb - 1023 - (FX_P - 1)) * (1 << 20);
   auto put = [&](auto ic, long long eq) {
     constexpr int I = decltype(ic)::value;
-    const long long x = mul_hi(q[I], a.fx[FX_OMC], eq);
+    const long long x = mul_hi_b(limbs(q[I]), a.fx[FX_OMC], eq);
     double r;
     if constexpr (I < fx_nint<L>) {
       r = fx_to_double(x, out20 + (1023 + Fx<L>::k(wclass<L>(I))) * (1 << 20));
@@ -250,37 +266,44 @@ __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inl
                            __double2loint(d));
     }
     if (store)
-      SF::template store<double, L>(fb + I * S + c, r, a.L.fbase[I], (unsigned)(cell * L::Q + I),
-                                    a.f16_sr);
+      SF::template store<double, L>(fb + a.doff[I] + at, r, a.L.fbase[I],
+                                    (unsigned)(cell * L::Q + I), a.f16_sr);
   };
+  auto pair = [&](auto kc, long long even, long long odd) {  // direction i and its opposite
+    constexpr int i = L::pair(decltype(kc)::value);
+    put(std::integral_constant<int, i>{}, even + odd);
+    put(std::integral_constant<int, L::opp(i)>{}, even - odd);
+  };
+  // pair index of velocity (x, y, z) or of its opposite; the odd part's sign
+  auto dir = [&](auto xc, auto yc, auto zc, long long even, long long odd) {
+    constexpr int i = dir_of<L>(decltype(xc)::value, decltype(yc)::value, decltype(zc)::value);
+    constexpr int k = pair_of<L>(i);
+    pair(std::integral_constant<int, k>{}, even, L::pair(k) == i ? odd : -odd);
+  };
+  using P1 = std::integral_constant<int, 1>;
+  using N1 = std::integral_constant<int, -1>;
+  using Z0 = std::integral_constant<int, 0>;
   put(std::integral_constant<int, 0>{}, G);
-  static_for(
-      [&](auto kc) {
-        constexpr int k = decltype(kc)::value;
-        constexpr int i = L::pair(k), j = L::opp(L::pair(k));
-        constexpr int ex = L::ex(i), ey = L::ey(i), ez = L::ez(i);
-        long long even = G, odd = 0;
-        if constexpr (ex != 0) {
-          even += qd[0];
-          odd = ex > 0 ? v[0] : -v[0];
-        }
-        if constexpr (ey != 0) {
-          even += qd[1];
-          odd = ey > 0 ? odd + v[1] : odd - v[1];
-        }
-        if constexpr (D == 3 && ez != 0) {
-          even += qd[D - 1];
-          odd = ez > 0 ? odd + v[D - 1] : odd - v[D - 1];
-        }
-        if constexpr (ex * ey != 0) even = ex * ey > 0 ? even + qo[0] : even - qo[0];
-        if constexpr (D == 3) {
-          if constexpr (ex * ez != 0) even = ex * ez > 0 ? even + qo[1] : even - qo[1];
-          if constexpr (ey * ez != 0) even = ey * ez > 0 ? even + qo[2] : even - qo[2];
-        }
-        put(std::integral_constant<int, i>{}, even + odd);
-        put(std::integral_constant<int, j>{}, even - odd);
-      },
-      std::make_integer_sequence<int, L::NPAIR>{});
+  const long long ex = G + qd[0], ey = G + qd[1], exy = ex + qd[1];
+  const long long vp = v[0] + v[1], vm = v[0] - v[1];
+  dir(P1{}, Z0{}, Z0{}, ex, v[0]);
+  dir(Z0{}, P1{}, Z0{}, ey, v[1]);
+  dir(P1{}, P1{}, Z0{}, exy + qo[0], vp);
+  dir(P1{}, N1{}, Z0{}, exy - qo[0], vm);
+  if constexpr (D == 3) {
+    const long long exz = ex + qd[2], eyz = ey + qd[2], e3 = exy + qd[2];
+    const long long sp = qo[1] + qo[2], sm = qo[1] - qo[2];  // 2 (Q_xz +- Q_yz)
+    dir(Z0{}, Z0{}, P1{}, G + qd[2], v[2]);
+    dir(P1{}, Z0{}, P1{}, exz + qo[1], v[0] + v[2]);
+    dir(P1{}, Z0{}, N1{}, exz - qo[1], v[0] - v[2]);
+    dir(Z0{}, P1{}, P1{}, eyz + qo[2], v[1] + v[2]);
+    dir(Z0{}, P1{}, N1{}, eyz - qo[2], v[1] - v[2]);
+    const long long ep = e3 + qo[0], em = e3 - qo[0];
+    dir(P1{}, P1{}, P1{}, ep + sp, vp + v[2]);
+    dir(P1{}, P1{}, N1{}, ep - sp, vp - v[2]);
+    dir(P1{}, N1{}, P1{}, em + sm, vm + v[2]);
+    dir(P1{}, N1{}, N1{}, em - sm, vm - v[2]);
+  }
   return true;
 }
 

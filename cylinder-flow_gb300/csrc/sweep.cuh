@@ -292,7 +292,7 @@ __device__ __forceinline__ void finish_cell(A *f, A rho3, A ux, A uy, A uz, long
                                             long long S, const SweepArgs &a) {
   if (a.mu && store) store_macros<A>(a, cell, rho3, ux, uy, uz);
   if (a.alpha) {
-    const A s = VA<A>::sub(A(1), static_cast<A>(a.alpha[cell]));
+    const A s = VA<A>::sub(A(1), store ? static_cast<A>(a.alpha[cell]) : A(0));
     ux = VA<A>::mul(ux, s);
     uy = VA<A>::mul(uy, s);
     uz = VA<A>::mul(uz, s);
@@ -323,7 +323,10 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_kernel(const 
   const int z = blockIdx.z;
   if (x >= a.L.nx || y >= a.L.ny) return;
   const long long S = a.L.S;
-  const long long c = a.L.idx(x, y, z);
+  // the block's first cell (uniform) and the thread's place from there
+  const long long c0 = a.L.idx(blockIdx.x * SWEEP_BX, blockIdx.y * SWEEP_BY, z);
+  const unsigned at = threadIdx.y * (unsigned)a.L.rs + threadIdx.x;
+  const long long c = c0 + at;
   const E *__restrict__ fa = static_cast<const E *>(a.fa);
   E *__restrict__ fb = static_cast<E *>(a.fb);
 
@@ -332,15 +335,14 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_kernel(const 
   A f[Q];
 #pragma unroll
   for (int i = 0; i < Q; ++i)
-    f[i] = SF::template load<A, L>(fa + i * S + c - a.L.off(L::ex(i), L::ey(i), L::ez(i)),
-                                   a.L.fbase[i]);
+    f[i] = SF::template load<A, L>(fa + c0 + a.poff[i] + at, a.L.fbase[i]);
   pdl_trigger();
 
   const long long cell = ((long long)z * a.L.ny + y) * a.L.nx + x;
   if constexpr (std::is_same<A, double>::value) {
     const bool in = a.ref_override && x == 0;
     if (fixed_cell<L, SF>(f, solid, in, in ? a.inlet_u[(long long)z * a.L.ny + y] : 0.0,
-                          a.ref_override && x == a.L.nx - 1, cell, true, fb, c, S, a))
+                          a.ref_override && x == a.L.nx - 1, cell, true, fb + c0, at, a))
       return;
   }
   A rho3, ux, uy, uz;
@@ -973,11 +975,15 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_channel_kerne
   const int y = by * SWEEP_BY + threadIdx.y;
   if (y >= ny) return;
   const int t = a.tile_index[((long long)z * ny + y) * a.nxw + blockIdx.x];
-  int x = blockIdx.x * SWEEP_BX + lane;
+  // The block's first cell (uniform) and the thread's place from there: one 32-bit
+  // offset for all populations.  Lanes past the last cell load padding and store
+  // nothing.
+  const int x = blockIdx.x * SWEEP_BX + lane;
   const bool valid = x < nx;
-  if (!valid) x = nx - 1;
   const long long S = a.L.S;
-  const long long c = a.L.idx(x, y, z);
+  const long long c0 = a.L.idx(blockIdx.x * SWEEP_BX, by * SWEEP_BY, z);
+  const unsigned at = threadIdx.y * (unsigned)a.L.rs + lane;
+  const long long c = c0 + at;
   const E *__restrict__ fa = static_cast<const E *>(a.fa);
   E *__restrict__ fb = static_cast<E *>(a.fb);
   A f[Q];
@@ -997,17 +1003,30 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_channel_kerne
         std::make_integer_sequence<int, Q>{});
   } else {
     pdl_wait();
+    // the plain pull; e_x < 0 from one element back, so that the outlet column can
+    // repeat itself without a negative offset
+    const unsigned am = at + (x == nx - 1 ? 0u : 1u);
     static_for(
         [&](auto ic) {
           constexpr int I = decltype(ic)::value;
-          f[I] = pull_plain<Q, ST, A, I>(fa, c, S, x, a);
+          constexpr bool back = DirC<Q, I>::ex < 0;
+          f[I] = SF::template load<A, L>(fa + (c0 - (back ? 1 : 0)) + a.poff[I] + (back ? am : at),
+                                         a.L.fbase[I]);
         },
         std::make_integer_sequence<int, Q>{});
+    if (blockIdx.x == 0) {  // the inlet column
+      static_for(
+          [&](auto ic) {
+            constexpr int I = decltype(ic)::value;
+            if constexpr (DirC<Q, I>::ex > 0) f[I] = x == 0 ? inlet_pop<A>(a, I) : f[I];
+          },
+          std::make_integer_sequence<int, Q>{});
+    }
   }
   const long long cell = ((long long)z * ny + y) * nx + x;
   pdl_trigger();
   if constexpr (std::is_same<A, double>::value) {
-    if (fixed_cell<L, SF>(f, solid_here, false, 0.0, false, cell, valid, fb, c, S, a)) return;
+    if (fixed_cell<L, SF>(f, solid_here, false, 0.0, false, cell, valid, fb + c0, at, a)) return;
   }
   A rho3, ux, uy, uz;
   moments<L, A, SF>(f, rho3, ux, uy, uz);

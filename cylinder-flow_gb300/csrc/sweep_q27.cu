@@ -5,11 +5,10 @@ namespace cflbm {
 
 cudaError_t launch_sweep_q27(int store, int compute, const SweepArgs &a, cudaStream_t s) {
   if (compute != COMPUTE_F32) {
-    // Block fixed point (fixed.cuh): 5 blocks per SM (96 registers).  REF3D
-    // 257x97x97, 20 steps and the fields: 5.51 / 5.46 ms at 5 / 6 per SM (6 spills
-    // 130 bytes); FP64 operations at 3 per SM: 15.17 ms.
+    // Block fixed point (fixed.cuh).  REF3D 257x97x97, 20 steps and the fields: 4.83 /
+    // 4.64 ms at 5 / 6 blocks per SM; FP64 operations at 3 per SM: 15.17 ms.
     switch (store) {
-      case STORE_F64: return launch_sweep_t<27, double, double, 5>(a, s);
+      case STORE_F64: return launch_sweep_t<27, double, double, 6>(a, s);
       case STORE_F32: return launch_sweep_t<27, float, double, 5>(a, s);
       case STORE_F16: return launch_sweep_t<27, F16Dev, double, 5>(a, s);
     }
@@ -26,8 +25,8 @@ cudaError_t launch_sweep_q27(int store, int compute, const SweepArgs &a, cudaStr
 cudaError_t launch_sweep_channel_q27(int store, int compute, const SweepArgs &a,
                                       cudaStream_t s) {
   if (compute != COMPUTE_F32) {
-    // Block fixed point: 512x128x128, 10 steps and the fields: 9.67 / 8.39 / 8.55 ms
-    // at 4 / 5 / 6 per SM; FP64 operations at 3 per SM: 22.78 ms.
+    // Block fixed point: 512x128x128, 10 steps and the fields: 7.33 / 7.81 ms at 5 / 6
+    // per SM; FP64 operations at 3 per SM: 22.78 ms.
     switch (store) {
       case STORE_F64: return launch_sweep_channel_t<27, double, double, 5>(a, s);
       case STORE_F32: return launch_sweep_channel_t<27, float, double, 5>(a, s);

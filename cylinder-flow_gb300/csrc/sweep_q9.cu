@@ -23,8 +23,8 @@ cudaError_t launch_sweep_q9(int store, int compute, const SweepArgs &a, cudaStre
 cudaError_t launch_sweep_channel_q9(int store, int compute, const SweepArgs &a,
                                      cudaStream_t s) {
   if (compute != COMPUTE_F32) {
-    // Block fixed point: 1132x168, 400 steps 3.48 / 3.48 / 3.36 ms at 4 / 6 / 8
-    // blocks per SM; 400x100 1.91 / 1.91 / 1.92.
+    // Block fixed point: 1132x168, 400 steps 3.32 / 3.22 ms at 7 / 8 blocks per
+    // SM; 400x100 1.78 / 1.79.
     switch (store) {
       case STORE_F64: return launch_sweep_channel_t<9, double, double, 8>(a, s);
       case STORE_F32: return launch_sweep_channel_t<9, float, double, 4>(a, s);
