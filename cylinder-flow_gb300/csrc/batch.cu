@@ -7,8 +7,7 @@
 // Each instance is an ordinary channel-profile handle (its own buffers, mask,
 // solid-tile list, force history), so every per-instance result call of the C ABI
 // works on cflbm_batch_handle(b, k).  The batch adds:
-//   * a device table of per-instance sweep arguments, one per A/B parity and
-//     macro flag;
+//   * a device table of per-instance sweep arguments, one per A/B parity;
 //   * a work list of (instance, tile block) items for the interior launch, each
 //     carrying its warp tiles' unlisted flags, and one for the solid-tile launch
 //     (blocks of `by` listed tiles of one instance);
@@ -38,10 +37,12 @@ struct cflbm_batch {
   int Q = 9, storage = 0, compute = 1;
   cudaStream_t stream = nullptr;
   int device = 0;
-  SweepArgs *d_args = nullptr;       // [inst][parity][macros]
+  SweepArgs *d_args = nullptr;       // [inst][parity]
   int4 *d_work_fast[4] = {nullptr};  // per tile height candidate index
   int4 *d_work_solid[4] = {nullptr};
   int n_work_fast[4] = {0}, n_work_solid[4] = {0};
+  int4 *d_work_force = nullptr;  // (instance, force block)
+  int n_work_force = 0;
   int by = 4;            // tuned tile height
   int grid = 0;          // tuned persistent grid size
   int sms = 152;
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(32 * BY, SOLID ? 16 / BY + 1 : 24 / BY)
     if (w + 1 < w1) wn = work[w + 1];
     if (wk.x != staged) {     // block-uniform
       __syncthreads();
-      const int *src = reinterpret_cast<const int *>(args + 4 * (long long)wk.x + sel);
+      const int *src = reinterpret_cast<const int *>(args + 2 * (long long)wk.x + sel);
       int *dst = reinterpret_cast<int *>(&a);
       for (int k = tid; k < (int)(sizeof(SweepArgs) / sizeof(int)); k += 32 * BY) dst[k] = src[k];
       __syncthreads();
@@ -213,48 +214,85 @@ __global__ void __launch_bounds__(32 * BY, SOLID ? 16 / BY + 1 : 24 / BY)
   }
 }
 
-// Fast items, one per block: the block reads its item and its instance's
-// arguments straight from global memory (cached in L1; no shared-memory staging
-// and no barrier), and the hardware scheduler keeps the SMs full.  The launch
-// is latency-bound, so it is held to 48 registers (40 warps per SM, no spill);
-// measured on the 64-channel problem: 0.889 of the copy peak against 0.822 at
-// 59 registers and 0.881 at 40 registers (a 24-byte spill).
-template <int Q, class ST, int BY, int MINB = 40 / BY>
+// One step as one launch, started while the step before still runs: the force blocks
+// of every instance, its listed tiles (BY per block), then the fast items, one per
+// block.  A block reads its item and its instance's arguments straight from global
+// memory (cached in L1; no shared-memory staging and no barrier), and the hardware
+// scheduler keeps the SMs full.  The launch is latency-bound, so it is held to 48
+// registers (40 warps per SM, no spill); measured on the 64-channel problem: 0.889 of
+// the copy peak against 0.822 at 59 registers and 0.881 at 40 registers (a 24-byte
+// spill).  With the listed tiles and the force on a persistent grid beside it, 200
+// steps of that problem took 17.4 ms, so 16.5; 24 channels of 300-1800 x 64-250 0.058 ->
+// 0.054 ms per step; six D3Q27 channels (96 registers there) 0.147 -> 0.095.
+template <int Q, class ST, int BY, int MINB = (Q == 9 ? 40 : 20) / BY>
 __global__ void __launch_bounds__(32 * BY, MINB)
-    batch_fast_kernel(const SweepArgs *__restrict__ args, const int4 *__restrict__ work, int sel) {
-  const int4 wk = work[blockIdx.x];  // (instance, x pair | row flags << 16, y tile, z)
-  const SweepArgs &a = args[4 * (long long)wk.x + sel];
-  const int wid = threadIdx.y;
+    batch_step_kernel(const SweepArgs *__restrict__ args, const int4 *__restrict__ force, int nf,
+                      const int4 *__restrict__ solid, int ns, const int4 *__restrict__ work,
+                      int sel) {
+  pdl_trigger();
+  const int b = blockIdx.x, wid = threadIdx.y, lane = threadIdx.x;
+  if (b < nf) {
+    const int4 wk = force[b];  // (instance, block of the instance, 0, 0)
+    const SweepArgs &a = args[2 * (long long)wk.x + sel];
+    force_cells<Q, ST, float, true, BY>(a, wk.y, a.bnd_blocks);
+    return;
+  }
+  if (b < nf + ns) {
+    const int4 wk = solid[b - nf];  // (instance, 0, listed block, 0)
+    const SweepArgs &a = args[2 * (long long)wk.x + sel];
+    const long long t = (long long)wk.z * BY + wid;
+    if (t >= a.n_slow) return;  // warp-uniform
+    const int tile = a.slow_tiles[t], row = tile / a.nxw;
+    const unsigned links = a.links_bits[t * 32 + lane];
+    pdl_wait();
+    channel_listed_cell<Q, ST, float>(a, (tile - row * a.nxw) * 32 + lane, row % a.L.ny,
+                                      row / a.L.ny, links);
+    return;
+  }
+  const int4 wk = work[b - nf - ns];  // (instance, x pair | row flags << 16, y tile, z)
+  const SweepArgs &a = args[2 * (long long)wk.x + sel];
   const unsigned rf = ((unsigned)wk.y >> 16) >> (2 * wid);
   const bool act0 = rf & 1u, act1 = (rf >> 1) & 1u;
+  pdl_wait();
   if (act0 || act1)  // warp-uniform
-    channel2_cells<Q, ST, float2, false, false>(a, 64 * (wk.y & 0xffff) + threadIdx.x,
-                                                wk.z * BY + wid, wk.w, act0, act1);
+    channel2_cells<Q, ST, float2, false, false>(a, 64 * (wk.y & 0xffff) + lane, wk.z * BY + wid,
+                                                wk.w, act0, act1);
 }
 
-// grid > 0: persistent grids of `grid` blocks for both kinds of work; grid = 0:
-// one fast item per block, and the solid work on 8 warps per SM.
+template <int Q, class ST, int BY>
+cudaError_t launch_batch_step_t(const cflbm_batch *b, int sel, cudaStream_t s) {
+  const int ci = BY == 1 ? 0 : BY == 2 ? 1 : BY == 4 ? 2 : 3;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(b->n_work_force + b->n_work_solid[ci] + b->n_work_fast[ci]));
+  cfg.blockDim = dim3(32, BY, 1);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(
+      &cfg, batch_step_kernel<Q, ST, BY>, (const SweepArgs *)b->d_args,
+      (const int4 *)b->d_work_force, b->n_work_force, (const int4 *)b->d_work_solid[ci],
+      b->n_work_solid[ci], (const int4 *)b->d_work_fast[ci], sel);
+  count_launch();
+  return e == cudaSuccess ? cudaGetLastError() : e;
+}
+
+// Persistent grids of `grid` blocks for both kinds of work (kind 0: interior items,
+// 1: listed tiles and force).
 template <int Q, class ST, int BY>
 cudaError_t launch_batch_t(const cflbm_batch *b, int kind, int sel, int grid, cudaStream_t s) {
   const int ci = BY == 1 ? 0 : BY == 2 ? 1 : BY == 4 ? 2 : 3;
   dim3 block(32, BY, 1);
   if (kind == 0) {
-    if (b->n_work_fast[ci] > 0) {
-      if (grid > 0)
-        batch_sweep_kernel<Q, ST, float, BY, false>
-            <<<std::min(grid, b->n_work_fast[ci]), block, 0, s>>>(b->d_args, b->d_work_fast[ci],
-                                                                  b->n_work_fast[ci], sel);
-      else
-        batch_fast_kernel<Q, ST, BY><<<b->n_work_fast[ci], block, 0, s>>>(
-            b->d_args, b->d_work_fast[ci], sel);
-    }
+    if (b->n_work_fast[ci] > 0)
+      batch_sweep_kernel<Q, ST, float, BY, false>
+          <<<std::min(grid, b->n_work_fast[ci]), block, 0, s>>>(b->d_args, b->d_work_fast[ci],
+                                                                b->n_work_fast[ci], sel);
   } else {
-    // Beside one-item-per-block interior launches: 8 solid warps per SM
-    // (64-channel problem, tile height 2: 0.889 of the copy peak at 4 blocks
-    // per SM against 0.769 at 2; tile height 4: 0.880 at 2 blocks per SM).
-    const int g = grid > 0 ? grid : std::max(1, 8 / BY) * b->sms;
     batch_sweep_kernel<Q, ST, float, BY, true>
-        <<<std::max(1, std::min(g, b->n_work_solid[ci])), block, 0, s>>>(
+        <<<std::max(1, std::min(grid, b->n_work_solid[ci])), block, 0, s>>>(
             b->d_args, b->d_work_solid[ci], b->n_work_solid[ci], sel);
   }
   count_launch();
@@ -264,6 +302,12 @@ cudaError_t launch_batch_t(const cflbm_batch *b, int kind, int sel, int grid, cu
 template <int Q, class ST>
 cudaError_t launch_batch_st(const cflbm_batch *b, int by, int kind, int sel, int grid,
                             cudaStream_t s) {
+  if (kind == 2) switch (by) {  // a whole step
+    case 1: return launch_batch_step_t<Q, ST, 1>(b, sel, s);
+    case 2: return launch_batch_step_t<Q, ST, 2>(b, sel, s);
+    case 4: return launch_batch_step_t<Q, ST, 4>(b, sel, s);
+    default: return launch_batch_step_t<Q, ST, 8>(b, sel, s);
+  }
   switch (by) {
     case 1: return launch_batch_t<Q, ST, 1>(b, kind, sel, grid, s);
     case 2: return launch_batch_t<Q, ST, 2>(b, kind, sel, grid, s);
@@ -284,18 +328,22 @@ cudaError_t launch_batch(const cflbm_batch *b, int by, int kind, int sel, int gr
   return launch_batch_st<27, F16Dev>(b, by, kind, sel, grid, s);
 }
 
-// One batch step: both launches, reading buffer `parity` of every instance.  The
-// solid-work kernel (tiles next to a body or on a wall row; latency-bound, with
-// the force reduction) runs on the higher-priority side stream beside the fast
-// kernel; the two write disjoint cells.
-int batch_one_step(cflbm_batch *b, int by, int grid, bool macros, bool swap) {
-  const int sel = b->parity * 2 + (macros ? 1 : 0);
-  BCK(cudaEventRecord(b->fork.fork, b->stream));
-  BCK(cudaStreamWaitEvent(b->fork.side, b->fork.fork, 0));
-  BCK(launch_batch(b, by, 1, sel, grid, b->fork.side));
-  BCK(cudaEventRecord(b->fork.join, b->fork.side));
-  BCK(launch_batch(b, by, 0, sel, grid, b->stream));
-  BCK(cudaStreamWaitEvent(b->stream, b->fork.join, 0));
+// One batch step, reading buffer `parity` of every instance.  grid = 0: one launch.
+// grid > 0: persistent grids, the solid-work kernel (tiles next to a body or on a wall
+// row; latency-bound, with the force reduction) on the higher-priority side stream
+// beside the fast kernel; the two write disjoint cells.
+int batch_one_step(cflbm_batch *b, int by, int grid, bool swap) {
+  const int sel = b->parity;
+  if (grid == 0) {
+    BCK(launch_batch(b, by, 2, sel, 0, b->stream));
+  } else {
+    BCK(cudaEventRecord(b->fork.fork, b->stream));
+    BCK(cudaStreamWaitEvent(b->fork.side, b->fork.fork, 0));
+    BCK(launch_batch(b, by, 1, sel, grid, b->fork.side));
+    BCK(cudaEventRecord(b->fork.join, b->fork.side));
+    BCK(launch_batch(b, by, 0, sel, grid, b->stream));
+    BCK(cudaStreamWaitEvent(b->stream, b->fork.join, 0));
+  }
   if (swap) {
     b->parity ^= 1;
     ++b->steps_done;
@@ -310,6 +358,7 @@ void free_batch(cflbm_batch *b) {
   for (auto g : b->graph)
     if (g) cudaGraphExecDestroy(g);
   if (b->d_args) cudaFree(b->d_args);
+  if (b->d_work_force) cudaFree(b->d_work_force);
   for (int k = 0; k < 4; ++k) {
     if (b->d_work_fast[k]) cudaFree(b->d_work_fast[k]);
     if (b->d_work_solid[k]) cudaFree(b->d_work_solid[k]);
@@ -390,15 +439,24 @@ int cflbm_batch_create(const cflbm_config *cfgs, int n, const cflbm_batch_option
   }
   const int es = b->storage == CFLBM_STORE_FP64 ? 8 : b->storage == CFLBM_STORE_FP32 ? 4 : 2;
   b->bytes_per_cell = 2.0 * b->Q * es + 0.125;
-  // Per-instance arguments: [parity][macros].
-  std::vector<SweepArgs> args((size_t)n * 4);
+  // Per-instance arguments: [parity].
+  std::vector<SweepArgs> args((size_t)n * 2);
+  std::vector<int4> wforce;
   for (int k = 0; k < n; ++k) {
     cflbm_handle *h = b->inst[k];
-    for (int par = 0; par < 2; ++par)
-      for (int m = 0; m < 2; ++m)
-        args[(size_t)k * 4 + par * 2 + m] =
-            channel_args(h, h->buf[par], h->buf[par ^ 1], m == 1);
+    // up to 512 boundary cells in one block: its sum needs no partials
+    const int nb = h->n_bcells <= 512 ? 1 : h->args.bnd_blocks;
+    for (int q = 0; q < nb; ++q) wforce.push_back(make_int4(k, q, 0, 0));
+    for (int par = 0; par < 2; ++par) {
+      SweepArgs &sa = args[(size_t)k * 2 + par];
+      sa = channel_args(h, h->buf[par], h->buf[par ^ 1], false);
+      sa.bnd_blocks = nb;
+    }
   }
+  b->n_work_force = (int)wforce.size();
+  BCK(cudaMalloc(&b->d_work_force, wforce.size() * sizeof(int4)));
+  BCK(cudaMemcpy(b->d_work_force, wforce.data(), wforce.size() * sizeof(int4),
+                 cudaMemcpyHostToDevice));
   BCK(cudaMalloc(&b->d_args, args.size() * sizeof(SweepArgs)));
   BCK(cudaMemcpy(b->d_args, args.data(), args.size() * sizeof(SweepArgs), cudaMemcpyHostToDevice));
   // Per-tile listed flags of every instance, read back once.
@@ -456,10 +514,10 @@ int cflbm_batch_create(const cflbm_config *cfgs, int n, const cflbm_batch_option
         const int by = BY_CANDIDATES[ci];
         if (32 * by * bps > 2048) continue;
         const int grid = bps * sms;
-        int rc = batch_one_step(b, by, grid, false, false);
+        int rc = batch_one_step(b, by, grid, false);
         if (rc) return rc;
         BCK(cudaEventRecord(e0, b->stream));
-        for (int r = 0; r < 5 && rc == CFLBM_OK; ++r) rc = batch_one_step(b, by, grid, false, false);
+        for (int r = 0; r < 5 && rc == CFLBM_OK; ++r) rc = batch_one_step(b, by, grid, false);
         if (rc) return rc;
         BCK(cudaEventRecord(e1, b->stream));
         BCK(cudaEventSynchronize(e1));
@@ -506,7 +564,7 @@ int cflbm_batch_step(cflbm_batch *b, int nsteps) {
       BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
       int rc = CFLBM_OK;
       for (int s = 0; s < b->graph_steps && rc == CFLBM_OK; ++s)
-        rc = batch_one_step(b, b->by, b->grid, false, true);
+        rc = batch_one_step(b, b->by, b->grid, true);
       cudaError_t ec = cudaStreamEndCapture(b->stream, &g);
       if (rc) {
         if (g) cudaGraphDestroy(g);
@@ -520,12 +578,12 @@ int cflbm_batch_step(cflbm_batch *b, int nsteps) {
       b->steps_done -= b->graph_steps;
     }
     BCK(cudaGraphLaunch(b->graph[b->parity], b->stream));
-    count_launch(2LL * b->graph_steps);
+    count_launch((b->grid == 0 ? 1LL : 2LL) * b->graph_steps);
     b->steps_done += b->graph_steps;
     left -= b->graph_steps;
   }
   for (int s = 0; s < left; ++s) {
-    int rc = batch_one_step(b, b->by, b->grid, s == left - 1, true);
+    int rc = batch_one_step(b, b->by, b->grid, true);
     if (rc) return rc;
   }
   // Keep the instance handles' host state in step with the device.
@@ -533,6 +591,11 @@ int cflbm_batch_step(cflbm_batch *b, int nsteps) {
     h->fA = h->buf[b->parity];
     h->fB = h->buf[b->parity ^ 1];
     h->steps_done = b->steps_done;
+    // u, v, w, p are formed on request, as for a single channel
+    if (nsteps > 0) {
+      h->macros_pending = true;
+      h->macros_direct = false;
+    }
   }
   return publish(b);
 }

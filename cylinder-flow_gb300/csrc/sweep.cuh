@@ -781,9 +781,9 @@ __device__ __forceinline__ void channel2_cells(const SweepArgs &a, int x0, int y
 // warp shuffles, per block, and over blocks, in block order, by the last block to
 // finish, into the force-history slot of this step.  One block alone needs no
 // partials and no counter.
+template <int NW>
 __device__ __forceinline__ void force_to_history(const SweepArgs &a, double dx, double dy,
                                                  double dz, unsigned blk, unsigned nblk) {
-  constexpr int NW = SWEEP_BY;
   const int lane = threadIdx.x, wid = threadIdx.y;
   const int tid = wid * SWEEP_BX + lane;
   __shared__ double sh[3][NW];
@@ -835,7 +835,7 @@ __device__ __forceinline__ void force_to_history(const SweepArgs &a, double dx, 
     __threadfence();
     const volatile double *p = a.partials;
     dx = dy = dz = 0.0;
-    for (unsigned k = tid; k < nblk; k += SWEEP_BX * SWEEP_BY) {
+    for (unsigned k = tid; k < nblk; k += SWEEP_BX * NW) {
       dx += p[3 * k];
       dy += p[3 * k + 1];
       dz += p[3 * k + 2];
@@ -855,15 +855,15 @@ __device__ __forceinline__ void force_to_history(const SweepArgs &a, double dx, 
 // populations the sweep bounces back (f*_{opp(I)}(X) from the state it pulls
 // from); per cell the sum runs in the arithmetic type, over cells in FP64.  PDL:
 // the first cells' list entries are read ahead of the predecessor's end.
-template <int Q, class ST, class A, bool PDL>
+template <int Q, class ST, class A, bool PDL, int NW = SWEEP_BY>
 __device__ __forceinline__ void force_cells(const SweepArgs &a, unsigned blk, unsigned nblk) {
   using L = Lat<Q>;
   using SF = Store<ST>;
   using E = typename SF::elem;
   const long long S = a.L.S;
   const E *__restrict__ fa = static_cast<const E *>(a.fa);
-  const int stride = (int)nblk * SWEEP_BX * SWEEP_BY;
-  int k = ((int)blk * SWEEP_BY + threadIdx.y) * SWEEP_BX + threadIdx.x;
+  const int stride = (int)nblk * SWEEP_BX * NW;
+  int k = ((int)blk * NW + threadIdx.y) * SWEEP_BX + threadIdx.x;
   unsigned links = 0;
   long long c = 0;
   if (k < a.n_bcells) {
@@ -900,7 +900,7 @@ __device__ __forceinline__ void force_cells(const SweepArgs &a, unsigned blk, un
       c = a.bcell_idx[k];
     }
   }
-  force_to_history(a, dx, dy, dz, blk, nblk);
+  force_to_history<NW>(a, dx, dy, dz, blk, nblk);
 }
 
 // The force as a launch of its own: with the line-staged sweep, and where the
