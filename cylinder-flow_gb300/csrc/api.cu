@@ -660,8 +660,8 @@ void set_relax(SweepArgs &a, int Q, int, double omega) {
     fix(FX_T, 0x1p63L * (4.5L * W * om));
     fix(FX_V, (Q == 27 ? 0x1p60L : 0x1p59L) * (3.0L * W * om));
     fix(FX_G, 0x1p61L * (W * om));
-    fix(FX_THIRD, 0x1p64L / 3.0L);
   }
+  fix(FX_THIRD, 0x1p64L / 3.0L);
 }
 
 void set_offsets(SweepArgs &a, int Q) {

@@ -29,7 +29,7 @@ cudaError_t launch_setup_list(const SetupArgs &s, const unsigned char *flag, con
                               int *list, uint32_t *links_bits, cudaStream_t st);
 
 // The boundary cells (fluid cells with solid links) of the listed tiles, in
-// tile and then x order, for the force launch: per listed tile its count
+// tile and then x order, for the force: per listed tile its count
 // (cnt: n_slow bytes; chunk: bcell_chunks(n_slow) + 1 ints; their number into
 // *total), then the storage index and link word of each.
 int bcell_chunks(int n_slow);

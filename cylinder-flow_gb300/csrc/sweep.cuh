@@ -28,7 +28,7 @@
 //                            and their solid links from per-cell link words, so
 //                            the branch adds one select per direction, not the
 //                            per-cell wall logic of pull_resolved.
-//   channel_force_kernel  -- beside the sweep on a second stream: the body force
+//   force_cells           -- the leading blocks of the sweeps: the body force
 //                            from the populations the sweep bounces back.
 //   macros_channel_kernel -- u, v, w, p on request.
 #pragma once
@@ -1042,7 +1042,7 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_channel_kerne
 // doubles per cell, straight into the caller's arrays; bound by HBM.  The pulls
 // are the sweep's: plain for unlisted tiles, the face-state tables for listed
 // ones.  Measured, macros_device at 768x384x384 FP16 / 512x128x128 FP32 / FP64 /
-// D2Q9 8192x1024 FP32: 2.3 / 0.20 / 0.69 / 0.13 ms against 7.5 / 0.56 / 1.05 / 0.22
+// D2Q9 8192x1024 FP32: 2.3 / 0.20 / 0.40 / 0.13 ms against 7.5 / 0.56 / 1.05 / 0.22
 // with the resolved pull for every cell, one cell per thread, and copies from the
 // handle's fields.  Two cells per thread at 5 / 6 / 8 blocks per SM: no difference.
 template <int Q, class ST, class A>
@@ -1206,7 +1206,7 @@ cudaError_t launch_macros_channel_t(const SweepArgs &a, cudaStream_t s) {
     const dim3 g2((a.nxw + 1) / 2, grid.y, grid.z);
     macros_channel2_kernel<Q, ST, Q == 9 ? 8 : 6><<<g2, block, 0, s>>>(a);
   } else {
-    macros_channel_kernel<Q, ST, A, 5><<<grid, block, 0, s>>>(a);
+    macros_channel_kernel<Q, ST, A, 6><<<grid, block, 0, s>>>(a);
   }
   count_launch();
   return cudaGetLastError();
