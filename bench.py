@@ -5,15 +5,15 @@ grid (D = 32 cells, axis along z through (128, 64)), equilibrium inlet
 u = (0.04, 0, 0), zero-gradient outlet, free-slip y, periodic z, Re = 200
 (tau = 0.5 + 3 u D / Re = 0.5192), initial rho = 1, uniform u plus a seeded
 +-1e-3 u_y perturbation.  The headline stores FP64 populations and computes in
-FP64, the reference's arithmetic (GB300's FP64 units run at ~1.2 TFLOP/s, so
-this form is bound by them, not by HBM).  The other forms -- double-float
-collision on FP64 storage, FP32 collision on FP64 / FP32 storage, FP16
+FP64, the reference's precision (the collision in block fixed point: GB300's FP64
+units issue two lanes per clock and SM).  The other forms -- DF64 (the same
+sweeps), FP32 collision on FP64 / FP32 storage, FP16
 deviation storage, both layouts -- are measured on the same grid under `forms`,
 each with its error after a few steps against the FP64 oracle's run of the
 same steps.
 
-One step = one time step of the whole grid (fused sweep + the body-force
-launch beside it).  `value` = interior cells x timed steps / device time
+One step = one time step of the whole grid (one launch: the fused sweep with the
+body force in it).  `value` = interior cells x timed steps / device time
 (MLUPS), inputs resident; the sweep time of the same steps comes from events
 around every sweep launch on the solver's stream; `e2e` = the same metric
 through the C ABI end to end: create the handle from host buffers (page-locked
@@ -322,9 +322,10 @@ def run_gb300(args):
                      "traffic": traffic, "peak_source": peak_kind,
                      "bytes_per_cell": info.bytes_per_cell_step,
                      "sweep_us": round(sweep_s * 1e6, 2),
-                     "note": "FP64 arithmetic is bound by GB300's FP64 units, not HBM: "
-                             "133 FP64 instructions per cell at 85 % FP64-pipe activity "
-                             "(ncu, profiles/sweep_instruction_mix_d3q27.md)"},
+                     "note": "FP64 precision in block fixed point: the FP64 pipe (32 "
+                             "conversions per cell, 69 % active) and the integer pipe "
+                             "(61 %) bind together "
+                             "(ncu, profiles/sweep_fp64_fixed_d3q27.md)"},
         "e2e": {"value": round(e2e_value, 2), "unit": "MLUPS", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "steps": e2e_steps, "forces_read_back": forces_ok,
                 "create_ms": round(1e3 * (t_created - t0), 2)},

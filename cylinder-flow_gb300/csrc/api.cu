@@ -1041,7 +1041,12 @@ int cflbm_forces(cflbm_handle *h, double fxyz[3], double cd_cl[2]) {
       // a caller that asks for forces: from the next step on through pinned memory
       // (without it the copy below, through pageable memory, goes on serving)
       void *p = nullptr;
-      if (cudaHostAlloc(&p, 64, cudaHostAllocMapped) == cudaSuccess) {
+      // (a capture that some thread has open allows this allocation)
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      const cudaError_t ea = cudaHostAlloc(&p, 64, cudaHostAllocMapped);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      if (ea == cudaSuccess) {
         h->force_host = static_cast<volatile double *>(p);
         void *d = nullptr;
         if (cudaHostGetDevicePointer(&d, p, 0) == cudaSuccess)
