@@ -199,9 +199,10 @@ __device__ __forceinline__ void fx_store_macros(const SweepArgs &a, long long ce
 
 // Collision and store of one cell with FP64 arithmetic, population i to
 // fb[doff_i + at] (fb: the block's first cell).  f: the pulled populations.  solid: p = u = 0; inlet: u = (ux_in, 0, 0); outlet: p = 0 (the
-// reference profiles' rules).  Returns false, with nothing written, where the
+// reference profiles' rules).  MACROS: fields out, where the step wants them.
+// Returns false, with nothing written, where the
 // format does not cover the cell.
-template <class L, class SF, class E>
+template <class L, class SF, bool MACROS, class E>
 __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inlet, double ux_in,
                                            bool outlet, long long cell, bool store,
                                            E *__restrict__ fb, unsigned at,
@@ -221,7 +222,8 @@ __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inl
   }
   if (outlet) mr = 0;
 
-  if (a.mu && store) fx_store_macros<L>(a, cell, eb, mr, mu);
+  if constexpr (MACROS)
+    if (a.mu && store) fx_store_macros<L>(a, cell, eb, mr, mu);
   if (a.alpha) {  // u (1 - alpha): the factor at 2^62, the product back by 4
     const Limbs sl = limbs(__double2ll_rn(__dmul_rn(s, 4611686018427387904.0)));
 #pragma unroll
