@@ -907,6 +907,14 @@ class PageMapper {
  public:
   PageMapper(void *p, size_t bytes) : p_(static_cast<char *>(p)), bytes_(bytes) {
     if (bytes < (8u << 20)) return;
+    // ordinary host memory only: pinned memory is mapped, other pointers are for the
+    // copies to take or to refuse
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return;
     try {
       done_ = std::vector<std::atomic<char>>((bytes + PIECE - 1) / PIECE);
       const unsigned n = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));

@@ -18,12 +18,13 @@ E27 = [(0, 0, 0)] + [s for p in [(1, 0, 0), (0, 1, 0), (0, 0, 1), (1, 1, 0), (1,
                      for s in (p, tuple(-v for v in p))]
 
 
-def one_step(f, E, w, omega):
+def one_step(f, E, w, omega, damp=1):
     """(next state, pulled state) of a periodic box in extended precision."""
     g = np.stack([np.roll(f[i], e[::-1], (0, 1, 2)) for i, e in enumerate(E)]).astype(np.longdouble)
     rho3 = g.sum(axis=0)
     u = [sum(e[d] * gi for e, gi in zip(E, g) if e[d]) for d in range(3)]
     u = [c if isinstance(c, np.ndarray) else 0 * rho3 for c in u]
+    u = [damp * c for c in u]
     usq = sum(c * c for c in u)
     out = []
     for i, e in enumerate(E):
@@ -94,3 +95,30 @@ def test_infinities_and_nans_spread_as_in_fp64(cuda, lattice, dims):
     bad = ~np.isfinite(g).all(axis=0)
     ok = np.isfinite(got).all(axis=0)
     assert bad.sum() == 2 and (~ok == bad).all()
+
+
+@pytest.mark.parametrize("lattice,dims", [(9, (67, 48, 1)), (27, (67, 32, 9))])
+def test_one_step_error_with_porosity(cuda, lattice, dims):
+    """Brinkman factors 1 - alpha inside [-1, 1] stay in the format (one more rounding,
+    a quarter unit), others take FP64 operations."""
+    from cflbm import Solver
+    E = E9 if lattice == 9 else E27
+    w = np.array([(np.longdouble(4) / 9 if lattice == 9 else np.longdouble(8) / 27)
+                  / np.longdouble(4) ** sum(map(abs, e)) for e in E])
+    nx, ny, nz = dims
+    f = states(E, w, (nz, ny, nx))
+    alpha = np.random.default_rng(6).choice([0.0, 0.3, 0.999, 1.0, 2.0, -0.5, 2.5], size=(nz, ny, nx))
+    alpha = alpha.astype(np.float32).astype(np.float64)
+    with Solver(lattice=lattice, nx=nx, ny=ny, nz=nz, tau0=0.03, u0=0.04, wall_y="periodic",
+                wall_z="periodic", geom="none", alpha=alpha) as s:
+        s.set_f(f, steps_done=0)
+        s.step(1)
+        got = s.get_f().reshape(f.shape)
+    ref, g = one_step(f, E, w, 1.0 / 0.53, np.longdouble(1) - alpha.astype(np.longdouble))
+    ins = (slice(None), slice(None), slice(1, nx - 1))
+    scale = np.abs(g / w.reshape(-1, 1, 1, 1)).max(axis=0)
+    err = np.abs((got - ref) / w.reshape(-1, 1, 1, 1)).max(axis=0).astype(float)
+    inside = (scale < 0.2 * (27 if lattice == 27 else 9)) & (np.abs(1 - alpha) <= 1)
+    tol = np.where(inside, 13.0, 64.0 * (1.0 + 2.25 * scale)) * 2.0 ** -53 * scale
+    tol = np.maximum(tol, 2.0 ** -940).astype(float)
+    assert (err[ins] <= tol[ins]).all(), float((err[ins] / tol[ins]).max())
