@@ -454,7 +454,7 @@ def run_channel2d(args):
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
                      "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": None,
                      "peak_source": peak_kind, "bytes_per_cell": bpc,
-                     "note": "L2-resident and launch-bound: two launches per step"},
+                     "note": "L2-resident and latency-bound: one launch per step"},
         "e2e": e2e, "gpu_launches": n_launch, "clocks": clk.summary(), "forms": forms,
         "cpu_baseline": cpu,
     }
