@@ -105,7 +105,8 @@ __device__ __forceinline__ int fx_exponent(const double *f, double ux) {
   // |ux| <= 8 max |g| keeps its integer below 2^62
   int hi = (__double2hiint(ux) & 0x7FFFFFFF) - (3 << 20);
 #pragma unroll
-  for (int c = 0; c <= L::D; ++c) hi = max(hi, __float_as_int(m[c]) - Fx<L>::k(c) * (1 << 20));
+  for (int c = 0; c <= L::D; ++c)  // NaNs as infinity: the shift stays below 2^31
+    hi = max(hi, min(__float_as_int(m[c]), 0x7F800000) - Fx<L>::k(c) * (1 << 20));
   return max(hi >> 20, FX_EMIN);
 }
 

@@ -1,0 +1,75 @@
+"""Values at the edges of the block fixed-point format: what is not finite or far out
+of it in any one population.
+"""
+import numpy as np
+import pytest
+
+from test_gpu_fixed_point import E9, E27
+
+pytestmark = pytest.mark.gpu
+
+BAD = (np.nan, np.inf, -np.inf, 1e307)
+
+
+def weights(lattice):
+    E = E9 if lattice == 9 else E27
+    return E, np.array([(np.longdouble(4) / 9 if lattice == 9 else np.longdouble(8) / 27)
+                        / np.longdouble(4) ** sum(map(abs, e)) for e in E])
+
+
+def pulled(f, E):
+    return np.stack([np.roll(f[i], e[::-1], (0, 1, 2)) for i, e in enumerate(E)])
+
+
+@pytest.mark.parametrize("storage,compute", [("fp64", "fp64"), ("fp64", "df64"), ("fp32", "fp64")])
+@pytest.mark.parametrize("lattice,dims", [(9, (64, 16, 1)), (27, (64, 16, 8))])
+def test_bad_value_in_any_one_population(cuda, lattice, dims, storage, compute):
+    """Every (population, value) has a cell of its own; the same cells are finite as in
+    FP64 arithmetic, populations and fields."""
+    from cflbm import Solver
+    E, w = weights(lattice)
+    nx, ny, nz = dims
+    f = np.full((len(E), nz, ny, nx), 1e-3)
+    bad = BAD if storage == "fp64" else BAD[:3]
+    for k, (i, v) in enumerate((i, v) for i in range(len(E)) for v in bad):
+        e = E[i]
+        x, y, z = 3 + 2 * (k % 28), 2 * (k // 28) + 1, k % nz
+        f[i, (z - e[2]) % nz, (y - e[1]) % ny, x - e[0]] = v
+    with Solver(lattice=lattice, nx=nx, ny=ny, nz=nz, tau0=0.02, u0=0.04, wall_y="periodic",
+                wall_z="periodic", geom="none", storage=storage, compute=compute) as s:
+        s.set_f(f, steps_done=0)
+        s.step(1)
+        got = s.get_f().reshape(f.shape)
+        mac = [np.asarray(m).reshape(f.shape[1:]) for m in s.macros()]
+    with np.errstate(all="ignore"):
+        g = pulled(f, E)
+        rho3 = g.sum(axis=0)
+        u = [sum((e[d] * gi for e, gi in zip(E, g) if e[d]), np.zeros_like(rho3)) for d in range(3)]
+        eu = [sum(e[d] * u[d] for d in range(3)) for e in E]
+        usq = sum(c * c for c in u)
+        feq = [float(wi) * (rho3 + 3 * a + 4.5 * a * a - 1.5 * usq) for wi, a in zip(w, eu)]
+        ref = g - (g - np.stack(feq)) / 0.52
+    ins = (Ellipsis, slice(1, nx - 1))
+    assert (~np.isfinite(g)).any(axis=0).sum() == 3 * len(E)
+    assert np.array_equal(np.isfinite(got)[ins], np.isfinite(ref)[ins])
+    for m, r in zip(mac, u + [rho3 / 3]):
+        assert np.array_equal(np.isfinite(m)[ins], np.isfinite(r)[ins])
+
+
+@pytest.mark.parametrize("storage", ["fp64", "fp32", "fp16dev"])
+@pytest.mark.parametrize("lattice,dims", [(9, (40, 9, 1)), (27, (40, 9, 5))])
+def test_domain_sums_report_a_bad_value_in_any_population(cuda, lattice, dims, storage):
+    from cflbm import Solver
+    nx, ny, nz = dims
+    with Solver(lattice=lattice, nx=nx, ny=ny, nz=nz, tau0=0.02, u0=0.04, geom="none", storage=storage,
+                compute="fp64" if storage == "fp64" else "fp32") as s:
+        f0 = s.get_f().reshape((lattice, nz, ny, nx))
+        for i in range(lattice):
+            for v in BAD[:3]:
+                f = f0.copy()
+                f[i, nz // 2, 4, 21] = v
+                s.set_f(f)
+                with pytest.raises(Exception):
+                    s.mass()
+        s.set_f(f0)
+        assert abs(s.mass()[0] - nx * ny * nz) < 1.0
