@@ -233,7 +233,7 @@ __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inl
 
   // Q_ab and V_a in units of 2^(E - 54).
   const int n = min(2 * Fx<L>::U - 9 + 1023 - eb, 63);
-  const long long half = (1LL << n) >> 1;
+  const long long half = (long long)((1ULL << n) >> 1);
   long long qd[D], qo[D == 3 ? 3 : 1], v[D];
   {
     Limbs ml[D], tl[D];

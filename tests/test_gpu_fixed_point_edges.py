@@ -1,5 +1,5 @@
 """Values at the edges of the block fixed-point format: what is not finite or far out
-of it in any one population.
+of it in any one population, and exact zeros.
 """
 import numpy as np
 import pytest
@@ -73,3 +73,27 @@ def test_domain_sums_report_a_bad_value_in_any_population(cuda, lattice, dims, s
                     s.mass()
         s.set_f(f0)
         assert abs(s.mass()[0] - nx * ny * nz) < 1.0
+
+
+@pytest.mark.parametrize("compute", ["fp64", "df64"])
+@pytest.mark.parametrize("lattice,dims", [(9, (67, 20, 1)), (27, (67, 12, 9))])
+def test_zeros_stay_zeros(cuda, lattice, dims, compute):
+    """A fluid at rest and the inside of a body; and cells of zeros beside others."""
+    from cflbm import Solver
+    E, _ = weights(lattice)
+    nx, ny, nz = dims
+    with Solver(lattice=lattice, nx=nx, ny=ny, nz=nz, tau0=0.02, u0=0.0, wall_y="noslip", wall_z="freeslip",
+                geom="cylinder", cx=20, cy=ny / 2.0, diam=6, compute=compute) as s:
+        f = np.zeros((lattice, nz, ny, nx))
+        s.set_f(f, steps_done=0)
+        s.step(3)
+        assert not s.get_f().any() and not any(np.asarray(m).any() for m in s.macros())
+    f = np.random.default_rng(3).normal(size=f.shape) * 1e-3
+    f[..., ny // 2:, :] = 0.0
+    with Solver(lattice=lattice, nx=nx, ny=ny, nz=nz, tau0=0.02, u0=0.0, wall_y="periodic",
+                wall_z="periodic", geom="none", compute=compute) as s:
+        s.set_f(f, steps_done=0)
+        s.step(1)
+        got = s.get_f().reshape(f.shape)
+    empty = ~pulled(f, E).any(axis=0)
+    assert empty.any() and not got[:, empty].any()
