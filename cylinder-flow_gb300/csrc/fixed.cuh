@@ -64,9 +64,9 @@ __device__ __forceinline__ Limbs limbs(long long x) {
 // their upper word needs no sign extension; callers take the FX_BIAS off once.
 constexpr long long FX_BIAS = 1LL << 31;
 __device__ __forceinline__ long long mul_hi_b(Limbs x, FxConst c, long long add) {
-  long long cross = (long long)x.l * c.h + (long long)0x8000000080000000ULL;
-  cross = (long long)x.h * c.l + cross;
-  return (long long)x.h * c.h + (add + (long long)((unsigned long long)cross >> 32));
+  unsigned long long cross = (unsigned long long)((long long)x.l * c.h) + 0x8000000080000000ULL;
+  cross += (unsigned long long)((long long)x.h * c.l);
+  return (long long)x.h * c.h + (add + (long long)(cross >> 32));
 }
 __device__ __forceinline__ long long mul_hi(Limbs x, FxConst c, long long add) {
   return mul_hi_b(x, c, add - FX_BIAS);
@@ -102,8 +102,8 @@ __device__ __forceinline__ int fx_exponent(const double *f, double ux) {
       },
       std::make_integer_sequence<int, L::NPAIR>{});
   m[0] = max_mag(0.0f, f[0], f[0]);
-  // |ux| <= 8 max |g| keeps its integer below 2^62
-  int hi = (__double2hiint(ux) & 0x7FFFFFFF) - (3 << 20);
+  // ux's integer, 2^(FX_P + U - E) ux, stays below 2^62
+  int hi = (__double2hiint(ux) & 0x7FFFFFFF) - ((6 - Fx<L>::U) << 20);
 #pragma unroll
   for (int c = 0; c <= L::D; ++c)  // NaNs as infinity: the shift stays below 2^31
     hi = max(hi, min(__float_as_int(m[c]), 0x7F800000) - Fx<L>::k(c) * (1 << 20));
@@ -209,7 +209,7 @@ __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inl
                                            E *__restrict__ fb, unsigned at,
                                            const SweepArgs &a) {
   constexpr int D = L::D;
-  const int eb = fx_exponent<L>(f, inlet && !solid ? ux_in : 0.0);
+  const int eb = fx_exponent<L>(f, inlet ? ux_in : 0.0);
   double s = 1.0;
   if (a.alpha && store) s = __dsub_rn(1.0, (double)a.alpha[cell]);
   if (!a.fx_ok || eb > FX_EMAX || !(fabs(s) <= 1.0)) return false;

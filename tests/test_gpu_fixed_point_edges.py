@@ -1,5 +1,6 @@
 """Values at the edges of the block fixed-point format: what is not finite or far out
-of it in any one population, and exact zeros.
+of it in any one population, exact zeros, and an inlet value far above its cell's
+populations.
 """
 import numpy as np
 import pytest
@@ -97,3 +98,25 @@ def test_zeros_stay_zeros(cuda, lattice, dims, compute):
         got = s.get_f().reshape(f.shape)
     empty = ~pulled(f, E).any(axis=0)
     assert empty.any() and not got[:, empty].any()
+
+
+@pytest.mark.parametrize("u0", [0.05, 0.0625 * (1 - 2.0 ** -40), 3.0])
+def test_inlet_value_far_above_its_cells(cuda, u0):
+    """The reference profiles' inlet column over zero populations, solid cells in it
+    included: omega feq(0, u_in).  16 roundings of the FP64 expression.  (Its end rows
+    pull the corner ghosts, which this variant never writes.)"""
+    from cflbm import Solver
+    E, w = weights(9)
+    w = w.astype(float)
+    with Solver(lattice=9, nx=8, ny=65, profile="ref2ds", tau0=0.03, u0=u0) as s:
+        assert s.solid().reshape(65, 8)[:, 0].any()
+        s.set_f(np.zeros((9, 1, 65, 8)), steps_done=0)
+        s.step(1)
+        got = s.get_f().reshape((9, 65, 8))[:, 1:-1, 0]
+        u = np.asarray(s.macros()[0]).reshape(65, 8)[1:-1, 0]
+    y = np.arange(1.0, 64.0)
+    uin = u0 * 4.0 * y * (64 - y) / 64.0 ** 2
+    ref = np.stack([w[i] * (3 * e[0] * uin + 4.5 * (e[0] * uin) ** 2 - 1.5 * uin ** 2)
+                    for i, e in enumerate(E)]) / 0.53
+    assert np.abs(got - ref).max() <= 16 * 2.0 ** -53 * np.abs(ref).max()
+    assert np.abs(u - uin).max() <= 4 * 2.0 ** -53 * u0
