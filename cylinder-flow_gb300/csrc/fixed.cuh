@@ -25,7 +25,8 @@
 //
 // Cells the format does not cover take the FP64 operations (bgk_relax_each):
 // |g_i| >= 1/4 (|u| well above 0.3), infinities and NaNs, and rates within 2^-20
-// of 0 or 2.  Below 2^-900 the exponent stays at -900.
+// of 2 or, with FP64 (not DF64) arithmetic, below 1.1 (D3Q27) or 0.69 (D2Q9) (see
+// set_relax).  Below 2^-900 the exponent stays at -900.
 #pragma once
 #include "solver.cuh"
 

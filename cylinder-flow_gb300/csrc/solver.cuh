@@ -205,9 +205,9 @@ cudaError_t launch_dense_rows(int Q, int store, const Layout &L, void *f, double
 cudaError_t launch_fill_value(int Q, int store, const Layout &L, void *f, cudaStream_t s);
 
 // Fill omega, omega_f and the relaxation constants rk/rkf and fx of a sweep for
-// lattice Q (any storage kind `store`: the codecs hand the arithmetic the
-// populations themselves).
-void set_relax(SweepArgs &a, int Q, int store, double omega);
+// lattice Q and arithmetic `compute` (ComputeKind; any storage: the codecs hand the
+// arithmetic the populations themselves).
+void set_relax(SweepArgs &a, int Q, int compute, double omega);
 // Fill doff/poff of a sweep from its layout a.L.
 void set_offsets(SweepArgs &a, int Q);
 

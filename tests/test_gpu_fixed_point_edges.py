@@ -1,11 +1,11 @@
 """Values at the edges of the block fixed-point format: what is not finite or far out
-of it in any one population, exact zeros, and an inlet value far above its cell's
-populations.
+of it in any one population, exact zeros, an inlet value far above its cell's
+populations, and slow relaxation.
 """
 import numpy as np
 import pytest
 
-from test_gpu_fixed_point import E9, E27
+from test_gpu_fixed_point import E9, E27, one_step
 
 pytestmark = pytest.mark.gpu
 
@@ -120,3 +120,27 @@ def test_inlet_value_far_above_its_cells(cuda, u0):
                     for i, e in enumerate(E)]) / 0.53
     assert np.abs(got - ref).max() <= 16 * 2.0 ** -53 * np.abs(ref).max()
     assert np.abs(u - uin).max() <= 4 * 2.0 ** -53 * u0
+
+
+@pytest.mark.parametrize("tau0", [3.0, 100.0, 1e6])
+@pytest.mark.parametrize("lattice,dims", [(9, (64, 20, 1)), (27, (64, 12, 5))])
+def test_slow_relaxation_keeps_small_populations(cuda, lattice, dims, tau0):
+    """At small omega a step moves a population by omega (feq - f): its error is a
+    rounding or two of its own value and omega times the 64 of the FP64 equilibrium."""
+    from cflbm import Solver
+    E, w = weights(lattice)
+    nx, ny, nz = dims
+    rng = np.random.default_rng(8)
+    f = 0.03 * rng.normal(size=(lattice, nz, ny, nx)) * w.reshape(-1, 1, 1, 1).astype(float)
+    f *= 10.0 ** -rng.integers(0, 12, size=f.shape)
+    with Solver(lattice=lattice, nx=nx, ny=ny, nz=nz, tau0=tau0, u0=0.04, wall_y="periodic",
+                wall_z="periodic", geom="none") as s:
+        s.set_f(f, steps_done=0)
+        s.step(1)
+        got = s.get_f().reshape(f.shape)
+    omega = 1.0 / (tau0 + 0.5)
+    ref, g = one_step(f, E, w, omega)
+    w = w.reshape(-1, 1, 1, 1).astype(float)
+    scale = w * np.abs(g / w).max(axis=0).astype(float)
+    tol = 2.0 ** -53 * (2 * np.abs(g).astype(float) + 64 * omega * scale)
+    assert (np.abs(got - ref).astype(float) <= tol)[..., 1:-1].all()
