@@ -183,6 +183,12 @@ cudaError_t launch_stream_state(int Q, int store, const SweepArgs &a, bool ref, 
 // Launch shape of the sweeps: blocks of 32 x 4 cells, one z plane per grid z
 // (the solid-tile launch runs 4 listed warp tiles per block).
 constexpr int SWEEP_BX = 32, SWEEP_BY = 4;
+// Rows of a block of the one-cell sweeps: they address a thread from the block's first
+// cell in 32 bits, and where SWEEP_BY rows need more (ROWS layout, from 1.6e8 columns
+// in D2Q9, 5.3e7 in D3Q27) a block takes one row.
+inline int sweep_rows(const Layout &L) {
+  return (SWEEP_BY - 1) * L.rs + SWEEP_BX < (1LL << 32) ? SWEEP_BY : 1;
+}
 cudaError_t launch_fill_channel(int Q, int store, const FillArgs &a, cudaStream_t s);
 // The face passes op[0..nops) of a step and, with la.blocks > 0, its link fill, as one
 // launch (both only where neither reads what the other writes).

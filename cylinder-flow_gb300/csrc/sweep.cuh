@@ -320,12 +320,12 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_kernel(const 
   using SF = Store<ST>;
   using E = typename SF::elem;
   const int x = blockIdx.x * SWEEP_BX + threadIdx.x;
-  const int y = blockIdx.y * SWEEP_BY + threadIdx.y;
+  const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int z = blockIdx.z;
   if (x >= a.L.nx || y >= a.L.ny) return;
   const long long S = a.L.S;
   // the block's first cell (uniform) and the thread's place from there
-  const long long c0 = a.L.idx(blockIdx.x * SWEEP_BX, blockIdx.y * SWEEP_BY, z);
+  const long long c0 = a.L.idx(blockIdx.x * SWEEP_BX, blockIdx.y * blockDim.y, z);
   const unsigned at = threadIdx.y * (unsigned)a.L.rs + threadIdx.x;
   const long long c = c0 + at;
   const E *__restrict__ fa = static_cast<const E *>(a.fa);
@@ -364,8 +364,9 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_kernel(const 
 
 template <int Q, class ST, class A, int MINB>
 cudaError_t launch_sweep_t(const SweepArgs &a, cudaStream_t s) {
-  dim3 block(SWEEP_BX, SWEEP_BY, 1);
-  dim3 grid((a.L.nx + SWEEP_BX - 1) / SWEEP_BX, (a.L.ny + SWEEP_BY - 1) / SWEEP_BY, a.L.nz);
+  const int by = sweep_rows(a.L);
+  dim3 block(SWEEP_BX, by, 1);
+  dim3 grid((a.L.nx + SWEEP_BX - 1) / SWEEP_BX, (a.L.ny + by - 1) / by, a.L.nz);
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
@@ -976,7 +977,7 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_channel_kerne
   const int lane = threadIdx.x;
   int by = blockIdx.y, z = blockIdx.z;
   if (force_block<Q, ST, A>(a, by, z)) return;
-  const int y = by * SWEEP_BY + threadIdx.y;
+  const int y = by * blockDim.y + threadIdx.y;
   if (y >= ny) return;
   const int t = a.tile_index[((long long)z * ny + y) * a.nxw + blockIdx.x];
   // The block's first cell (uniform) and the thread's place from there: one 32-bit
@@ -985,7 +986,7 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_channel_kerne
   const int x = blockIdx.x * SWEEP_BX + lane;
   const bool valid = x < nx;
   const long long S = a.L.S;
-  const long long c0 = a.L.idx(blockIdx.x * SWEEP_BX, by * SWEEP_BY, z);
+  const long long c0 = a.L.idx(blockIdx.x * SWEEP_BX, by * blockDim.y, z);
   const unsigned at = threadIdx.y * (unsigned)a.L.rs + lane;
   const long long c = c0 + at;
   const E *__restrict__ fa = static_cast<const E *>(a.fa);
@@ -1241,13 +1242,15 @@ cudaError_t launch_sweep_channel_t(const SweepArgs &a0, cudaStream_t s) {
     }
   }
   constexpr bool pair = sizeof(A) == 4 && !std::is_same<ST, double>::value;
-  dim3 grid(pair ? (a.nxw + 1) / 2 : a.nxw, (a.L.ny + SWEEP_BY - 1) / SWEEP_BY, a.L.nz);
+  const int by = pair ? SWEEP_BY : sweep_rows(a.L);
+  dim3 grid(pair ? (a.nxw + 1) / 2 : a.nxw, (a.L.ny + by - 1) / by, a.L.nz);
   // up to 4 boundary cells per thread in one block: its sum needs no partials
   if (a.bnd_blocks > 1 && a.n_bcells <= 4 * TB) a.bnd_blocks = 1;
   const int per = (int)(Q == 9 ? grid.x : grid.x * grid.y);
   a.force_span = (a.bnd_blocks + per - 1) / per;
   unsigned &span_dim = Q == 9 ? grid.y : grid.z;
-  if (span_dim + a.force_span > 65535u) {  // no room in the grid: a launch of its own
+  // no room in the grid, or blocks of one row: a launch of its own
+  if (a.force_span > 0 && (span_dim + a.force_span > 65535u || by != SWEEP_BY)) {
     channel_force_kernel<Q, ST, A, 4><<<a.bnd_blocks, dim3(SWEEP_BX, SWEEP_BY, 1), 0, s>>>(a);
     count_launch();
     a.force_span = 0;
@@ -1258,7 +1261,7 @@ cudaError_t launch_sweep_channel_t(const SweepArgs &a0, cudaStream_t s) {
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(SWEEP_BX, SWEEP_BY, 1);
+  cfg.blockDim = dim3(SWEEP_BX, by, 1);
   cfg.stream = s;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
