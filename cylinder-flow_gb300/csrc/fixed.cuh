@@ -106,8 +106,11 @@ __device__ __forceinline__ int fx_exponent(const double *f, double ux) {
   // ux's integer, 2^(FX_P + U - E) ux, stays below 2^62
   int hi = (__double2hiint(ux) & 0x7FFFFFFF) - ((6 - Fx<L>::U) << 20);
 #pragma unroll
-  for (int c = 0; c <= L::D; ++c)  // NaNs as infinity: the shift stays below 2^31
-    hi = max(hi, min(__float_as_int(m[c]), 0x7F800000) - Fx<L>::k(c) * (1 << 20));
+  for (int c = 0; c <= L::D; ++c) {
+    int h = __float_as_int(m[c]);
+    if (Fx<L>::k(c) < 0) h = min(h, 0x7F800000);  // NaNs as infinity: below 2^31 shifted
+    hi = max(hi, h - Fx<L>::k(c) * (1 << 20));
+  }
   return max(hi >> 20, FX_EMIN);
 }
 
