@@ -303,8 +303,8 @@ __global__ void __launch_bounds__(256) ref_boundary_kernel(const FillArgs a, con
   const FaceOp &op = ops.op[p];
   const int ta = op.axis == 0 ? 1 : 0, tb = op.axis == 2 ? 1 : 2;
   const int na = n[ta] + 2, nb = Q == 27 ? n[tb] + 2 : 1;
-  const int r = t - ops.start[p], k = r / (na * nb), rem = r - k * na * nb;
-  int i = (int)((op.dirs >> (5 * k)) & 31u);
+  const int r = t - ops.start[p], kr = r / (na * nb), rem = r - kr * na * nb;
+  int i = (int)((op.dirs >> (5 * (ops.first[p] + kr))) & 31u);
   PassCell g;
   g.c[2] = 0;
   const int pb = rem / na, pa = rem - pb * na - 1;
@@ -633,32 +633,38 @@ static void face_dirs(int Q, FaceOp &op) {
 }
 
 cudaError_t launch_ref_boundary(int Q, int store, const FillArgs &a, const FaceOp *op, int nops,
-                                const LinkArgs &la, cudaStream_t s) {
+                                const LinkArgs &la0, cudaStream_t s) {
+  LinkArgs la = la0;
   FaceOps ops{};
   ops.n = nops;
   const int n[3] = {a.L.nx, a.L.ny, a.L.nz};
+  long long cells[6] = {};
   for (int p = 0; p < nops; ++p) {
     ops.op[p] = op[p];
     face_dirs(Q, ops.op[p]);
     const int ta = op[p].axis == 0 ? 1 : 0, tb = op[p].axis == 2 ? 1 : 2;
-    const long long cells = (long long)(n[ta] + 2) * (Q == 27 ? n[tb] + 2 : 1);
-    const long long end = ops.start[p] + ops.op[p].ndir * cells;
-    if (end > 0x7fffffffLL) return cudaErrorInvalidValue;
-    ops.start[p + 1] = (int)end;
+    cells[p] = (long long)(n[ta] + 2) * (Q == 27 ? n[tb] + 2 : 1);
   }
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(la.blocks + (ops.start[nops] + 255) / 256));
-  cfg.blockDim = dim3(256);
-  cfg.stream = s;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaSuccess;
-  CFLBM_DISPATCH(Q, store, (e = cudaLaunchKernelEx(&cfg, ref_boundary_kernel<QQ, ST>, a, ops, la)));
-  count_launch();
-  return e == cudaSuccess ? cudaGetLastError() : e;
+  int p = 0, k = 0;
+  do {
+    if (!next_faces(ops, cells, FACE_THREADS, p, k)) return cudaErrorInvalidValue;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(la.blocks + (ops.start[nops] + 255) / 256));
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaSuccess;
+    CFLBM_DISPATCH(Q, store,
+                   (e = cudaLaunchKernelEx(&cfg, ref_boundary_kernel<QQ, ST>, a, ops, la)));
+    if (e != cudaSuccess) return e;
+    count_launch();
+    la.blocks = 0;  // the links go with the first
+  } while (p < nops);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_ghost_copy(int Q, int store, const Layout &L, const void *src, void *dst,

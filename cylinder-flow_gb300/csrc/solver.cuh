@@ -15,6 +15,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include "face_plan.hpp"
 #include "lattice.cuh"
 
 namespace cflbm {
@@ -129,22 +130,6 @@ struct FillArgs {
   const void *f_in;      // inlet equilibrium, Q stored elements (channel profile)
 };
 
-struct FaceOp {
-  int kind;  // 0 copy (inlet), 1 extrapolate (outlet), 2 bounce (wall)
-  int axis;  // 0 x, 1 y, 2 z
-  int side;  // 0 low, 1 high
-  int trim;  // 1: the pass skips the two ghost ends of its tangential range
-  int ndir;  // the populations the pass writes (filled by launch_ref_boundary),
-  unsigned long long dirs;  // 5 bits each, the k-th at bit 5k
-};
-
-// The passes of a step in their order; start: first thread of each.
-struct FaceOps {
-  int n;
-  int start[7];
-  FaceOp op[6];
-};
-
 struct LinkArgs {
   Layout L;
   void *f;
@@ -191,7 +176,8 @@ inline int sweep_rows(const Layout &L) {
 }
 cudaError_t launch_fill_channel(int Q, int store, const FillArgs &a, cudaStream_t s);
 // The face passes op[0..nops) of a step and, with la.blocks > 0, its link fill, as one
-// launch (both only where neither reads what the other writes).
+// launch (both only where neither reads what the other writes); several for faces
+// beyond FACE_THREADS.
 cudaError_t launch_ref_boundary(int Q, int store, const FillArgs &a, const FaceOp *op, int nops,
                                 const LinkArgs &la, cudaStream_t s);
 cudaError_t launch_ghost_copy(int Q, int store, const Layout &L, const void *src, void *dst,
