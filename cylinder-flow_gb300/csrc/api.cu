@@ -1,6 +1,5 @@
 // C ABI of the solver (include/cflbm.h): handle life cycle and the step loop.
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -8,12 +7,11 @@
 #include <cstring>
 #include <memory>
 #include <string>
-#include <exception>
 #include <thread>
 #include <vector>
-#include <unistd.h>
 #include <cuda.h>
 #include "handle.hpp"
+#include "page_map.hpp"
 #include "setup.cuh"
 
 using namespace cflbm;
@@ -905,65 +903,19 @@ static int ensure_macros(cflbm_handle *h) {
 }
 
 extern "C++" {
-// Maps the pages of a host buffer that is about to be overwritten, on several cores
-// ahead of the copies into it.  A dump into fresh memory was bound by the driver's
-// page faults on one core: 226 MB took 7.8-9.9 ms, 1.2 ms once the pages are there;
-// mapped by 8 cores just ahead of 32 MB copies 2.1 ms (4 cores 2.4; MADV_POPULATE_WRITE
-// on 4 / 8 cores, which contend for the address space, 3.9 / 6.7; a pinned bounce
-// buffer emptied by 8 / 12 cores 4.0 / 3.7).
-class PageMapper {
- public:
-  PageMapper(void *p, size_t bytes) : p_(static_cast<char *>(p)), bytes_(bytes) {
-    if (bytes < (8u << 20)) return;
-    // ordinary host memory only: pinned memory is mapped, other pointers are for the
-    // copies to take or to refuse
-    cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-      cudaGetLastError();
-      return;
-    }
-    if (at.type != cudaMemoryTypeUnregistered) return;
-    try {
-      done_ = std::vector<std::atomic<char>>((bytes + PIECE - 1) / PIECE);
-      const unsigned n = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
-      pool_.reserve(n);
-      for (unsigned t = 0; t < n; ++t) pool_.emplace_back([this] { work(); });
-    } catch (const std::exception &) {  // no more threads or memory: with what there is
-    }
-  }
-  ~PageMapper() {
-    next_ = done_.size();
-    for (auto &t : pool_) t.join();
-  }
-  // Returns when the first `upto` bytes are mapped.
-  void wait(size_t upto) {
-    if (pool_.empty()) return;
-    for (; ready_ < done_.size() && ready_ * PIECE < upto; ++ready_)
-      while (!done_[ready_].load(std::memory_order_acquire)) std::this_thread::yield();
-  }
-
- private:
-  static constexpr size_t PIECE = 2u << 20;
-  void work() {
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    for (size_t k; (k = next_.fetch_add(1)) < done_.size();) {
-      const size_t e = std::min(bytes_, (k + 1) * PIECE);
-      for (size_t o = k * PIECE; o < e; o += page) static_cast<volatile char *>(p_)[o] = 0;
-      static_cast<volatile char *>(p_)[e - 1] = 0;
-      done_[k].store(1, std::memory_order_release);
-    }
-  }
-  char *p_;
-  size_t bytes_, ready_ = 0;
-  std::atomic<size_t> next_{0};
-  std::vector<std::atomic<char>> done_;
-  std::vector<std::thread> pool_;
-};
+// Maps ahead the pages of a caller's buffer: ordinary host memory only; pinned memory
+// is mapped, other pointers are for the copies to take or to refuse.
+static void map_pages(PageMapper &map, void *p, size_t bytes) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) cudaGetLastError();
+  else if (at.type == cudaMemoryTypeUnregistered) map.start(p, bytes);
+}
 
 // Device to host, into memory that may not be mapped yet.
 constexpr size_t STAGE_BYTES = 32u << 20;
 cudaError_t copy_out(void *dst, const void *src, size_t bytes, cudaStream_t s) {
-  PageMapper map(dst, bytes);
+  PageMapper map;
+  map_pages(map, dst, bytes);
   cudaError_t e = cudaSuccess;
   for (size_t o = 0; o < bytes && e == cudaSuccess; o += STAGE_BYTES) {
     const size_t n = std::min(STAGE_BYTES, bytes - o);
@@ -1177,7 +1129,8 @@ int cflbm_get_f(cflbm_handle *h, double *out) {
   const size_t nx = h->L.nx, rows = (size_t)h->Q * h->L.ny * h->L.nz;
   size_t per = 0;
   if (int rc = stage_rows(h, nx * 8, rows, &per)) return rc;
-  PageMapper map(out, rows * nx * 8);
+  PageMapper map;
+  map_pages(map, out, rows * nx * 8);
   for (size_t r = 0; r < rows; r += per) {
     const size_t n = std::min(per, rows - r);
     CK_CUDA(launch_dense_rows(h->Q, h->cfg.storage, h->L, h->fA, h->d_stage, (long long)r,

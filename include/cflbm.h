@@ -189,7 +189,9 @@ int cflbm_mass(cflbm_handle *h, double *mass, double momentum[3]);
 
 /* Dump / restore the post-collision populations of the interior in FP64,
  * layout [i][z][y][x] (x fastest), q*nx*ny*nz doubles.  The reference has no
- * restart; this is the checkpoint path.  set_f also sets steps_done. */
+ * restart; this is the checkpoint path.  set_f also sets steps_done.  Where a call
+ * that fills host arrays (get_f, get_f_stream, macros) fails, their contents are
+ * unspecified. */
 int cflbm_get_f(cflbm_handle *h, double *out);
 int cflbm_set_f(cflbm_handle *h, const double *in, int64_t steps_done);
 
