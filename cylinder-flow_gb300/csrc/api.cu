@@ -758,7 +758,12 @@ static int one_step(cflbm_handle *h, bool last) {
     // u, v, w, p are formed on request (ensure_macros), not written every step;
     // `last`: the force also goes where cflbm_forces reads it.
     SweepArgs sa = channel_args(h, h->fA, h->fB, false);
-    if (last) sa.force_host = h->d_force_host;
+    if (last && h->d_force_host) {
+      // not in a caller's capture: its launches run later, or not at all
+      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+      CK_CUDA(cudaStreamIsCapturing(h->stream, &cs));
+      if (cs == cudaStreamCaptureStatusNone) sa.force_host = h->d_force_host;
+    }
     if (h->timing && (trc = record_event(h, &ts0))) return trc;
     CK_CUDA(launch_sweep_channel(Q, st, h->cfg.compute, sa, h->stream));
     if (h->timing) {
@@ -767,7 +772,7 @@ static int one_step(cflbm_handle *h, bool last) {
     }
     std::swap(h->fA, h->fB);
     ++h->steps_done;
-    if (last && h->d_force_host) h->force_host_step = h->steps_done;
+    if (sa.force_host) h->force_host_step = h->steps_done;
     h->macros_pending = true;
     h->macros_direct = false;
     return CFLBM_OK;
