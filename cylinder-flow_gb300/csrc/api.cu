@@ -983,6 +983,11 @@ int cflbm_macros_device(cflbm_handle *h, double *u, double *v, double *w, double
   if (h->macros_pending && !h->macros_direct) {
     bool ok = u || v || w || p;
     for (int k = 0; k < 4; ++k) ok = ok && (!dst[k] || kernel_writable(h, dst[k], N));
+    for (int k = 0; k < 4; ++k)  // arrays that overlap: the copies' order decides
+      for (int j = 0; j < k; ++j) {
+        const uintptr_t a = (uintptr_t)dst[j], b = (uintptr_t)dst[k];
+        ok = ok && (!a || !b || a + 8 * N <= b || b + 8 * N <= a);
+      }
     if (ok) {
       SweepArgs sa = channel_args(h, h->fB, nullptr, false);
       sa.mu = u;
