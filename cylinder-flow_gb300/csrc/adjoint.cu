@@ -28,6 +28,7 @@
 #include <cstring>
 #include <string>
 #include <vector>
+#include "float_limbs.hpp"
 #include "handle.hpp"
 
 namespace cflbm {
@@ -174,14 +175,14 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
   return s;
 }
 
-// Block sum of an FP32 value to FP64 accuracy without the FP64 pipe (two lanes per
-// SM: the shuffle tree of FP64 additions took 4 of the reverse step's 15 us at
-// 1024x256): every value as two integers over the block's largest exponent, 23
-// and 24 bits, whose sums over 128 threads are exact -- 2^-47 of the largest term.
+// Block sum of an FP32 value, at least as accurate as FP64 additions, without the FP64
+// pipe (two lanes per SM: the shuffle tree of FP64 additions took 4 of the reverse
+// step's 15 us at 1024x256): every value as three integers over the block's largest
+// exponent, whose sums over 128 threads are exact -- 2^-72 of the largest term.
 // Infinities, NaNs and blocks below 2^-86 take the FP64 tree.
 struct IntSums {
   unsigned top;
-  int hi, lo;
+  int a, b, c;
 };
 __device__ __forceinline__ double block_sum(float v, double *sh, IntSums &is) {
   const int tid = threadIdx.y * ABX + threadIdx.x;
@@ -192,18 +193,18 @@ __device__ __forceinline__ double block_sum(float v, double *sh, IntSums &is) {
   const int e = (int)(is.top >> 23);
   if (is.top == 0u) return 0.0;
   if (e < 40 || e == 255) return block_sum((double)v, sh);
-  // |v| < 2^(e - 126): |u| < 2^23
-  const float u = v * __uint_as_float((unsigned)(276 - e) << 23);
-  const int hi = __float2int_rn(u);
-  const int lo = __float2int_rn((u - (float)hi) * 16777216.0f);
-  const int shi = __reduce_add_sync(0xffffffffu, hi), slo = __reduce_add_sync(0xffffffffu, lo);
+  const FloatLimbs l = float_limbs(v, __uint_as_float((unsigned)(276 - e) << 23));
+  const int sa = __reduce_add_sync(0xffffffffu, l.a), sb = __reduce_add_sync(0xffffffffu, l.b),
+            sc = __reduce_add_sync(0xffffffffu, l.c);
   if ((tid & 31) == 0) {
-    atomicAdd(&is.hi, shi);
-    atomicAdd(&is.lo, slo);
+    atomicAdd(&is.a, sa);
+    atomicAdd(&is.b, sb);
+    atomicAdd(&is.c, sc);
   }
   __syncthreads();
   if (tid != 0) return 0.0;
-  return ((double)is.hi + (double)is.lo * (1.0 / 16777216.0)) *
+  constexpr double D = 1.0 / 16777216.0;
+  return ((double)is.a + ((double)is.b + (double)is.c * D) * D) *
          __hiloint2double((1023 + e - 149) << 20, 0);
 }
 __device__ __forceinline__ double block_sum(double v, double *sh, IntSums &) {
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(ANT, sizeof(A) == 4 ? 10 : 6) adjoint_kernel(c
   A al = A(0);
   if constexpr (!FINAL)
     if (a.alpha && aux != AUX_SOLID) al = A(a.alpha[cell]);
-  if (threadIdx.x == 0 && threadIdx.y == 0) is = {0u, 0, 0};
+  if (threadIdx.x == 0 && threadIdx.y == 0) is = {0u, 0, 0, 0};
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const A *mu_n = static_cast<const A *>(a.mu_next);
   const A *s = static_cast<const A *>(a.s);
