@@ -216,7 +216,8 @@ __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inl
   const int eb = fx_exponent<L>(f, inlet ? ux_in : 0.0);
   double s = 1.0;
   if (a.alpha && store) s = __dsub_rn(1.0, (double)a.alpha[cell]);
-  if (!a.fx_ok || eb > FX_EMAX || !(fabs(s) <= 1.0)) return false;
+  // (lanes that store nothing hold padding, which may be anything: never a reason)
+  if (!a.fx_ok || eb > FX_EMAX || !(fabs(s) <= 1.0)) return !store && a.fx_ok;
 
   long long q[L::Q], mr, mu[3];
   fx_moments<L>(f, eb, q, mr, mu);
