@@ -156,9 +156,28 @@ __device__ __forceinline__ float d2f_bits(double d) {
   return __uint_as_float(t | (hi & 0x80000000u));
 }
 
-// Storage codecs: load/store (global memory; ordinary cached loads, not the
-// read-only path: a kernel launched while its predecessor still writes the state
-// reads it after griddepcontrol.wait) and decode (an element already
+// Loads of the state: cached, and volatile, so that they stay behind the
+// griddepcontrol.wait (asm volatile too) of a kernel launched while its predecessor
+// still writes the state.  CUDA's __ldca of a binary16 is an asm that the compiler may
+// move across it; in that order of loads the FP16 D3Q27 step was also slower: 203.1 ->
+// 198.8 us at 512x128x128, 9.16 -> 8.42 at 100x40x36.
+__device__ __forceinline__ double ld_state(const double *p) {
+  double v;
+  asm volatile("ld.global.ca.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_state(const float *p) {
+  float v;
+  asm volatile("ld.global.ca.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ __half ld_state(const __half *p) {
+  unsigned short v;
+  asm volatile("ld.global.ca.b16 %0, [%1];" : "=h"(v) : "l"(p));
+  return __ushort_as_half(v);
+}
+
+// Storage codecs: load/store (global memory) and decode (an element already
 // read, e.g. from shared memory) convert between the stored element and the
 // arithmetic type A, so the arithmetic always sees the population itself.
 // `base` is the storage offset of the population (Layout::fbase): 0 for FP64 and
@@ -174,8 +193,8 @@ template <> struct Store<double> {
   }
   template <class A, class L>
   __device__ static A load(const elem *p, float) {
-    if constexpr (sizeof(A) == 4) return d2f_bits(__ldca(p));
-    else return static_cast<A>(__ldca(p));
+    if constexpr (sizeof(A) == 4) return d2f_bits(ld_state(p));
+    else return static_cast<A>(ld_state(p));
   }
   template <class A, class L>
   __device__ static void store(elem *p, A v, float, unsigned, bool) {
@@ -189,7 +208,7 @@ template <> struct Store<float> {
   template <class A>
   __device__ static A decode(elem v, float) { return static_cast<A>(v); }
   template <class A, class L>
-  __device__ static A load(const elem *p, float) { return static_cast<A>(__ldca(p)); }
+  __device__ static A load(const elem *p, float) { return static_cast<A>(ld_state(p)); }
   template <class A, class L>
   __device__ static void store(elem *p, A v, float, unsigned, bool) { *p = static_cast<float>(v); }
 };
@@ -251,7 +270,7 @@ template <> struct Store<F16Dev> {
     else return __fma_rn((double)h, 1.0 / F16_SCALE, (double)base);
   }
   template <class A, class L>
-  __device__ static A load(const elem *p, float base) { return decode<A>(__ldca(p), base); }
+  __device__ static A load(const elem *p, float base) { return decode<A>(ld_state(p), base); }
   template <class A, class L>
   __device__ static void store(elem *p, A v, float base, unsigned key, bool sr) {
     float sv;

@@ -646,11 +646,11 @@ __device__ __forceinline__ P pull_pair(const typename Store<ST>::elem *__restric
   else off = I * S - (Dd::ex + Dd::ey * rs + Dd::ez * zs);
   float r0 = 0.0f, r1 = 0.0f;
   if constexpr (Dd::ex < 0) {  // the outlet column repeats itself (pm = p - 1 there)
-    if (act0) r0 = PC::raw(__ldca(pm0 + off));
-    if (act1) r1 = PC::raw(__ldca(pm1 + off));
+    if (act0) r0 = PC::raw(ld_state(pm0 + off));
+    if (act1) r1 = PC::raw(ld_state(pm1 + off));
   } else {
-    if (act0) r0 = PC::raw(__ldca(p + off));
-    if (act1) r1 = PC::raw(__ldca(p + off + 32));
+    if (act0) r0 = PC::raw(ld_state(p + off));
+    if (act1) r1 = PC::raw(ld_state(p + off + 32));
   }
   const float b = a.L.fbase[I];
   float2 v = PC::dec(make_float2(r0, r1), make_float2(b, b));
@@ -670,7 +670,7 @@ __device__ __forceinline__ P pull_pair_listed(const typename Store<ST>::elem *__
   using PC = PairCodec<ST>;
   if constexpr (I == 0) {
     const float b = a.L.fbase[0];
-    return PC::dec(make_float2(PC::raw(__ldca(p)), act1 ? PC::raw(__ldca(p + 32)) : 0.0f),
+    return PC::dec(make_float2(PC::raw(ld_state(p)), act1 ? PC::raw(ld_state(p + 32)) : 0.0f),
                    make_float2(b, b));
   } else {
     const bool bb0 = wbb || ((l0 >> I) & 1u), bb1 = wbb || ((l1 >> I) & 1u);
@@ -682,8 +682,8 @@ __device__ __forceinline__ P pull_pair_listed(const typename Store<ST>::elem *__
     constexpr long long OS = Dd::opp;
     const float b0 = bb0 ? a.L.fbase[Dd::opp] : a.L.fbase[I];
     const float b1 = bb1 ? a.L.fbase[Dd::opp] : a.L.fbase[I];
-    const float r0 = PC::raw(__ldca(p + (bb0 ? a.doff[OS] : s0)));
-    const float r1 = act1 ? PC::raw(__ldca(p + (bb1 ? a.doff[OS] + 32 : s1))) : 0.0f;
+    const float r0 = PC::raw(ld_state(p + (bb0 ? a.doff[OS] : s0)));
+    const float r1 = act1 ? PC::raw(ld_state(p + (bb1 ? a.doff[OS] + 32 : s1))) : 0.0f;
     float2 v = PC::dec(make_float2(r0, r1), make_float2(b0, b1));
     if constexpr (Dd::ex > 0) v.x = (!bb0 && inlet0) ? a.f_in_f[I] : v.x;
     return v;
