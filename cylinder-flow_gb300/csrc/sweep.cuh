@@ -878,14 +878,22 @@ __device__ __forceinline__ void force_cells(const SweepArgs &a, unsigned blk, un
   if constexpr (PDL) pdl_wait();
   double dx = 0.0, dy = 0.0, dz = 0.0;
   while (k < a.n_bcells) {
+    // Every load ahead of the first conversion: a conversion after each one made the
+    // linked directions' loads a chain (D3Q27 100x40x36, FP64 storage and FP32
+    // arithmetic: 15.6 -> 12.1 us per step; FP16 8.45 -> 7.96).
+    E r[Q];
     A f[Q];
     static_for(
         [&](auto ic) {
           constexpr int I = decltype(ic)::value;
-          f[I] = ((links >> I) & 1u)
-                     ? SF::template load<A, L>(fa + (long long)DirC<Q, I>::opp * S + c,
-                                               a.L.fbase[DirC<Q, I>::opp])
-                     : A(0);
+          r[I] = E{};
+          if ((links >> I) & 1u) r[I] = ld_state(fa + (long long)DirC<Q, I>::opp * S + c);
+        },
+        std::make_integer_sequence<int, Q>{});
+    static_for(
+        [&](auto ic) {
+          constexpr int I = decltype(ic)::value;
+          f[I] = ((links >> I) & 1u) ? SF::template decode<A>(r[I], a.L.fbase[DirC<Q, I>::opp]) : A(0);
         },
         std::make_integer_sequence<int, Q>{});
     A Fx = A(0), Fy = A(0), Fz = A(0);
@@ -981,13 +989,16 @@ __global__ void __launch_bounds__(SWEEP_BX * SWEEP_BY, MINB) sweep_channel_kerne
   if (y >= ny) return;
   const int t = a.tile_index[((long long)z * ny + y) * a.nxw + blockIdx.x];
   // The block's first cell (uniform) and the thread's place from there: one 32-bit
-  // offset for all populations.  Lanes past the last cell load padding and store
-  // nothing.
-  const int x = blockIdx.x * SWEEP_BX + lane;
-  const bool valid = x < nx;
+  // offset for all populations.  Lanes past the last cell store nothing; they load that
+  // cell, or padding in FP64 arithmetic, which is not bound by its loads (331x101x90
+  // FP64 storage, FP32 arithmetic: padding 200.8, the cell 196.0 us per step; FP64
+  // arithmetic 512x128x128: 662 and 664).
+  const int xl = blockIdx.x * SWEEP_BX + lane;
+  const bool valid = xl < nx;
+  const int x = sizeof(A) == 4 ? min(xl, nx - 1) : xl;
   const long long S = a.L.S;
   const long long c0 = a.L.idx(blockIdx.x * SWEEP_BX, by * blockDim.y, z);
-  const unsigned at = threadIdx.y * (unsigned)a.L.rs + lane;
+  const unsigned at = threadIdx.y * (unsigned)a.L.rs + (unsigned)(sizeof(A) == 4 ? x - (int)blockIdx.x * SWEEP_BX : lane);
   const long long c = c0 + at;
   const E *__restrict__ fa = static_cast<const E *>(a.fa);
   E *__restrict__ fb = static_cast<E *>(a.fb);
@@ -1291,6 +1302,12 @@ cudaError_t launch_sweep_channel_t(const SweepArgs &a0, cudaStream_t s) {
       e = (long long)a.L.nx * a.L.ny >= (1LL << 20)
               ? launch(sweep_channel2_kernel<Q, ST, float2, 10, false>)
               : launch(sweep_channel2_kernel<Q, ST, float2, 5, true>);
+  } else if constexpr (Q == 9 && sizeof(A) == 4) {
+    // FP64 storage: 94.3 / 89.4 / 87.1 us per step at 8 / 10 / 12 blocks per SM on
+    // 4096x1024, 5.25 / 5.31 / 5.85 on 1021x241
+    e = (long long)a.L.nx * a.L.ny >= (1LL << 20)
+            ? launch(sweep_channel_kernel<Q, ST, A, 12>)
+            : launch(sweep_channel_kernel<Q, ST, A, MINB_FAST>);
   } else {
     e = launch(sweep_channel_kernel<Q, ST, A, MINB_FAST>);
   }

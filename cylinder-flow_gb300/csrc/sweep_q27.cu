@@ -34,7 +34,9 @@ cudaError_t launch_sweep_channel_q27(int store, int compute, const SweepArgs &a,
     }
   } else {
     switch (store) {
-      case STORE_F64: return launch_sweep_channel_t<27, double, float, 8>(a, s);
+      // 512x128x128: 525.9 / 523.8 / 527.4 us per step at 6 / 7 / 8 per SM, 331x101x90
+      // 197.7 / 194.5 / 195.9, 100x40x36 11.3 / 11.4 / 12.1
+      case STORE_F64: return launch_sweep_channel_t<27, double, float, 7>(a, s);
       case STORE_F32: return launch_sweep_channel_t<27, float, float, 8>(a, s);
       case STORE_F16: return launch_sweep_channel_t<27, F16Dev, float, 8>(a, s);
     }
