@@ -67,7 +67,7 @@ void free_handle(cflbm_handle *h) {
   void *ptrs[] = {h->fA,    h->fB,     h->d_mask, h->d_links, h->d_mu,      h->d_mv,
                   h->d_links_bits, h->d_tile_slow, h->d_slow_tiles, h->d_tile_index,
                   h->d_face_off, h->d_face_bb, h->d_bcell_idx, h->d_bcell_links,
-                  h->d_mw,  h->d_mp,   h->d_inlet, h->d_alpha, h->d_fin,    h->d_hist,
+                  h->d_mw,  h->d_mp,   h->d_inlet, h->d_alpha, h->d_hist,
                   h->d_step, h->d_partials, h->d_counter, h->d_counter2, h->d_sums,
                   h->d_err, h->d_stage};
   for (void *p : ptrs)
@@ -164,28 +164,6 @@ void face_tables(const Layout &Ly, int wall_y, int wall_z, std::vector<long long
       off[(size_t)st * Q + i] = (long long)j * Ly.S + src;
       if (b) bb[st] |= 1u << i;
     }
-}
-
-// Equilibrium of the channel inlet (p = 0, u = (u_in, 0, 0)) in storage format
-// (FP16: the deviation from the storage offset fbase, times F16_SCALE).
-template <int Q>
-std::vector<unsigned char> inlet_elements(double u_in, int storage, const float *fbase) {
-  using L = Lat<Q>;
-  std::vector<unsigned char> out((size_t)Q * store_size(storage));
-  for (int i = 0; i < Q; ++i) {
-    const double edu = L::ex(i) * u_in;
-    const double feq = L::w(i) * 0.0 * 3.0 + L::w(i) * (3.0 * edu + 4.5 * edu * edu - 1.5 * u_in * u_in);
-    if (storage == CFLBM_STORE_FP64) {
-      std::memcpy(&out[8 * i], &feq, 8);
-    } else if (storage == CFLBM_STORE_FP32) {
-      const float v = (float)feq;
-      std::memcpy(&out[4 * i], &v, 4);
-    } else {
-      const __half v = __double2half((feq - (double)fbase[i]) * (double)F16_SCALE);
-      std::memcpy(&out[2 * i], &v, 2);
-    }
-  }
-  return out;
 }
 
 // Storage offsets of the FP16 format: the free-stream equilibrium
@@ -508,10 +486,6 @@ int cflbm_create(const cflbm_config *cfg, cflbm_handle **out) {
   if (h->lines) CK_CUDA(lines_prepare());
 
   if (cfg->profile == CFLBM_PROFILE_CHANNEL) {
-    std::vector<unsigned char> fin = d3 ? inlet_elements<27>(cfg->u0, cfg->storage, L.fbase)
-                                        : inlet_elements<9>(cfg->u0, cfg->storage, L.fbase);
-    if ((rc = dev_alloc(h, &h->d_fin, fin.size()))) return rc;
-    CK_CUDA(cudaMemcpyAsync(h->d_fin, fin.data(), fin.size(), cudaMemcpyHostToDevice, h->stream));
     if (cfg->alpha) {
       std::vector<float> a(N);
       for (size_t n = 0; n < N; ++n) a[n] = (float)cfg->alpha[n];

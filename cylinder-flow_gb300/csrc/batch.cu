@@ -1,22 +1,20 @@
 // Batched channels: many independent channel instances of uneven size and
-// Reynolds number advanced together, one work-list launch per sweep kind per
-// step over all instances, replayed from a captured CUDA graph, with the launch
-// shape (tile height; one interior item per block or a persistent grid size)
-// picked by a timing autotuner at creation.
+// Reynolds number advanced together, one launch per step over all instances,
+// replayed from a captured CUDA graph, with the launch shape (tile height; one work
+// item per block or persistent grids) picked by a timing autotuner at creation.
 //
 // Each instance is an ordinary channel-profile handle (its own buffers, mask,
 // solid-tile list, force history), so every per-instance result call of the C ABI
 // works on cflbm_batch_handle(b, k).  The batch adds:
 //   * a device table of per-instance sweep arguments, one per A/B parity;
-//   * a work list of (instance, tile block) items for the interior launch, each
-//     carrying its warp tiles' unlisted flags, and one for the solid-tile launch
-//     (blocks of `by` listed tiles of one instance);
-//   * the interior kernels (one item per block, or a persistent grid walking
-//     contiguous ranges of items) and the persistent solid kernel, running the
-//     same per-cell code as the single-channel sweep (channel2_cells,
-//     pull_resolved, moments, finish_cell); the solid kernel reduces each
-//     instance's body force into that instance's history, the last block of the
-//     instance summing its partials in block order.
+//   * work lists of (instance, tile block) items for the interior, each carrying its
+//     warp tiles' unlisted flags, of blocks of `by` listed tiles of one instance, and
+//     of the force blocks of every instance;
+//   * the step kernel (batch_step_kernel: force blocks, listed tiles and interior items,
+//     one per block), and a variant on persistent grids (batch_sweep_kernel: interior
+//     items and listed tiles as two launches side by side, each walking contiguous
+//     ranges of items, the listed one reducing every instance's force).  Both run the
+//     per-cell code of the single-channel sweep.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -108,44 +106,35 @@ __global__ void __launch_bounds__(32 * BY, SOLID ? 16 / BY + 1 : 24 / BY)
       __syncthreads();
       staged = wk.x;
     }
-    const int nx = a.L.nx, ny = a.L.ny;
-    int x = 0, y = 0, z = 0;
-    bool active = false;
-    long long t = 0;
-    if constexpr (SOLID) {
-      t = (long long)wk.z * BY + wid;
-      active = t < a.n_slow;
-      const int tile = active ? a.slow_tiles[t] : 0;
-      const int row = tile / a.nxw;
-      y = row % ny;
-      z = row / ny;
-      x = (tile % a.nxw) * 32 + lane;
-    } else {
+    if constexpr (!SOLID) {
       // Bits 2r and 2r + 1 of the row flags: warp tiles 2 * pair and 2 * pair + 1
       // of row r of the item are unlisted (and inside the box).
-      y = wk.z * BY + wid;
-      z = wk.w;
       const int pair = wk.y & 0xffff;
       const unsigned rf = ((unsigned)wk.y >> 16) >> (2 * wid);
       const bool act0 = rf & 1u, act1 = (rf >> 1) & 1u;
       if (act0 || act1)  // warp-uniform
-        channel2_cells<Q, ST, float2, false, false>(a, 64 * pair + lane, y, z, act0, act1);
-      continue;
-    }
-    double Fx = 0.0, Fy = 0.0, Fz = 0.0;
-    if (active) {  // warp-uniform
-      const bool valid = x < nx;
-      if (!valid) x = nx - 1;
-      const long long S = a.L.S;
-      const long long c = a.L.idx(x, y, z);
-      const E *__restrict__ fa = static_cast<const E *>(a.fa);
-      E *__restrict__ fb = static_cast<E *>(a.fb);
-      A f[Q];
-      bool solid_here = false;
-      A Fxa = A(0), Fya = A(0), Fza = A(0);
-      if constexpr (SOLID) {
+        channel2_cells<Q, ST, float2, false, false>(a, 64 * pair + lane, wk.z * BY + wid, wk.w,
+                                                    act0, act1);
+    } else {
+      const int nx = a.L.nx, ny = a.L.ny;
+      const long long t = (long long)wk.z * BY + wid;
+      const bool active = t < a.n_slow;
+      const int tile = active ? a.slow_tiles[t] : 0;
+      const int row = tile / a.nxw;
+      const int y = row % ny, z = row / ny;
+      int x = (tile % a.nxw) * 32 + lane;
+      double Fx = 0.0, Fy = 0.0, Fz = 0.0;
+      if (active) {  // warp-uniform
+        const bool valid = x < nx;
+        if (!valid) x = nx - 1;
+        const long long S = a.L.S;
+        const long long c = a.L.idx(x, y, z);
+        const E *__restrict__ fa = static_cast<const E *>(a.fa);
+        E *__restrict__ fb = static_cast<E *>(a.fb);
+        A f[Q];
+        A Fxa = A(0), Fya = A(0), Fza = A(0);
         const unsigned links = a.links_bits[t * 32 + lane];
-        solid_here = mask_solid(a.mask, a.nxw, ny, x, y, z);
+        const bool solid_here = mask_solid(a.mask, a.nxw, ny, x, y, z);
         static_for(
             [&](auto ic) {
               constexpr int I = decltype(ic)::value;
@@ -156,23 +145,14 @@ __global__ void __launch_bounds__(32 * BY, SOLID ? 16 / BY + 1 : 24 / BY)
         Fx = f2d_bits(Fxa);
         Fy = f2d_bits(Fya);
         Fz = f2d_bits(Fza);
-      } else {
-        static_for(
-            [&](auto ic) {
-              constexpr int I = decltype(ic)::value;
-              f[I] = pull_plain<Q, ST, A, I>(fa, c, S, x, a);
-            },
-            std::make_integer_sequence<int, Q>{});
+        A rho3, ux, uy, uz;
+        moments<L, A, SF>(f, rho3, ux, uy, uz);
+        if (solid_here) {
+          rho3 = A(0); ux = A(0); uy = A(0); uz = A(0);
+        }
+        const long long cell = ((long long)z * ny + y) * nx + x;
+        finish_cell<L, SF, A, E>(f, rho3, ux, uy, uz, cell, valid, fb, c, S, a);
       }
-      A rho3, ux, uy, uz;
-      moments<L, A, SF>(f, rho3, ux, uy, uz);
-      if (solid_here) {
-        rho3 = A(0); ux = A(0); uy = A(0); uz = A(0);
-      }
-      const long long cell = ((long long)z * ny + y) * nx + x;
-      finish_cell<L, SF, A, E>(f, rho3, ux, uy, uz, cell, valid, fb, c, S, a);
-    }
-    if constexpr (SOLID) {
       __shared__ double sh[3][BY];
       __shared__ bool last;
       for (int o = 16; o > 0; o >>= 1) {

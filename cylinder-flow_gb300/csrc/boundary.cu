@@ -3,7 +3,6 @@
 // These run on O(surface) work (ghost layers, fluid->solid links) except the
 // initialisation, reduction and dump/restore kernels, which run once or on
 // demand.  The hot per-step sweep is in sweep.cuh.
-#include <cstdio>
 #include "fixed.cuh"
 #include "solver.cuh"
 
@@ -38,16 +37,6 @@ template <int Q> __device__ int dopp(int i) { return Lat<Q>::opp(i); }
 template <> __device__ int dopp<9>(int i) {
   return i == 0 ? 0 : (i <= 4 ? (i + 1) % 4 + 1 : (i - 3) % 4 + 5);
 }
-template <int Q> __device__ int dmirror(int i, int d) {
-  int w0 = DT<Q>::ex(i), w1 = DT<Q>::ey(i), w2 = DT<Q>::ez(i);
-  if (d == 1) w1 = -w1;
-  if (d == 2) w2 = -w2;
-  if (d == 0) w0 = -w0;
-  for (int k = 0; k < Q; ++k)
-    if (DT<Q>::ex(k) == w0 && DT<Q>::ey(k) == w1 && DT<Q>::ez(k) == w2) return k;
-  return i;
-}
-
 // FP64 values of stored elements and back (Store<> codecs; L.fbase is the
 // FP16 format's storage offset per population).
 template <class ST> struct Dec;
@@ -77,79 +66,6 @@ inline int blocks_for(long long n, int threads) {
   if (b < 1) b = 1;
   if (b > 65535LL * 8) b = 65535LL * 8;
   return (int)b;
-}
-
-// ---- channel-profile ghost fill ------------------------------------------------
-// Post-stream value of direction i0 at interior cell X (pull from S = X - e_i0):
-//   z out of range: periodic wrap, or free-slip mirror (i := mirror_z(i),
-//   S.z := X.z), or no-slip (halfway bounce-back: f*_{opp(i0)}(X));
-//   then the same for y; then S.x < 0 -> inlet equilibrium, S.x >= nx -> x := nx-1
-//   (zero gradient); a solid source -> f*_{opp(i0)}(X).
-template <int Q, class E>
-__device__ E resolve_channel(const E *f, const FillArgs &a, int i0, int x, int y, int z) {
-  const Layout &L = a.L;
-  int i = i0;
-  int sx = x - DT<Q>::ex(i0), sy = y - DT<Q>::ey(i0), sz = z - DT<Q>::ez(i0);
-  if (Q == 27 && (sz < 0 || sz >= L.nz)) {
-    if (a.wall_z == WALL_PERIODIC) sz = (sz + L.nz) % L.nz;
-    else if (a.wall_z == WALL_FREESLIP) { i = dmirror<Q>(i, 2); sz = z; }
-    else return f[dopp<Q>(i0) * L.S + L.idx(x, y, z)];
-  }
-  if (sy < 0 || sy >= L.ny) {
-    if (a.wall_y == WALL_PERIODIC) sy = (sy + L.ny) % L.ny;
-    else if (a.wall_y == WALL_FREESLIP) { i = dmirror<Q>(i, 1); sy = y; }
-    else return f[dopp<Q>(i0) * L.S + L.idx(x, y, z)];
-  }
-  if (sx < 0) return static_cast<const E *>(a.f_in)[i];
-  if (sx >= L.nx) sx = L.nx - 1;
-  if (mask_solid(a.mask, a.nxw, L.ny, sx, sy, sz)) return f[dopp<Q>(i0) * L.S + L.idx(x, y, z)];
-  return f[i * L.S + L.idx(sx, sy, sz)];
-}
-
-template <int Q, class ST>
-__global__ void fill_channel_kernel(const FillArgs a) {
-  using E = typename Store<ST>::elem;
-  E *f = static_cast<E *>(a.f);
-  const Layout &L = a.L;
-  const bool d3 = (Q == 27);
-  const long long zr = d3 ? (L.nz + 2) : 1;
-  const long long nfx = (long long)(L.ny + 2) * zr;
-  const long long nfy = (long long)L.nx * zr;
-  const long long nfz = d3 ? (long long)L.nx * L.ny : 0;
-  const long long total = 2 * (nfx + nfy + nfz);
-  const int z0 = d3 ? -1 : 0;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    long long r = t;
-    int sx, sy, sz;
-    if (r < 2 * nfx) {
-      const int side = (int)(r / nfx);
-      r %= nfx;
-      sx = side ? L.nx : -1;
-      sy = (int)(r % (L.ny + 2)) - 1;
-      sz = (int)(r / (L.ny + 2)) + z0;
-    } else if ((r -= 2 * nfx) < 2 * nfy) {
-      const int side = (int)(r / nfy);
-      r %= nfy;
-      sy = side ? L.ny : -1;
-      sx = (int)(r % L.nx);
-      sz = (int)(r / L.nx) + z0;
-    } else {
-      r -= 2 * nfy;
-      const long long nfzd = nfz > 0 ? nfz : 1;
-      const int side = (int)(r / nfzd);
-      r %= nfzd;
-      sz = side ? L.nz : -1;
-      sx = (int)(r % L.nx);
-      sy = (int)(r / L.nx);
-    }
-    const long long sidx = L.idx(sx, sy, sz);
-    for (int i = 1; i < Q; ++i) {
-      const int X = sx + DT<Q>::ex(i), Y = sy + DT<Q>::ey(i), Z = sz + DT<Q>::ez(i);
-      if (!L.interior(X, Y, Z)) continue;
-      f[i * L.S + sidx] = resolve_channel<Q, E>(f, a, i, X, Y, Z);
-    }
-  }
 }
 
 // ---- solid links: bounce-back fill + momentum-exchange force ----------------
@@ -605,17 +521,6 @@ cudaError_t launch_sweep_channel(int Q, int store, int compute, const SweepArgs 
       else { using ST = F16Dev; CALL; }                                  \
     }                                                                    \
   } while (0)
-
-cudaError_t launch_fill_channel(int Q, int store, const FillArgs &a, cudaStream_t s) {
-  const bool d3 = Q == 27;
-  const long long zr = d3 ? a.L.nz + 2 : 1;
-  const long long total = 2 * ((a.L.ny + 2) * zr + (long long)a.L.nx * zr +
-                               (d3 ? (long long)a.L.nx * a.L.ny : 0));
-  const int blocks = blocks_for(total, 128);
-  CFLBM_DISPATCH(Q, store, (fill_channel_kernel<QQ, ST><<<blocks, 128, 0, s>>>(a)));
-  count_launch();
-  return cudaGetLastError();
-}
 
 // The populations a pass writes: e along its axis positive (inlet copy, low wall)
 // or negative (outlet extrapolation, high wall) -- 9 in D3Q27, 3 in D2Q9.

@@ -42,7 +42,6 @@ struct cflbm_handle {
   double *d_mu = nullptr, *d_mv = nullptr, *d_mw = nullptr, *d_mp = nullptr;
   double *d_inlet = nullptr;
   float *d_alpha = nullptr;
-  void *d_fin = nullptr;
   double *d_hist = nullptr;
   long long hist_cap = 0;
   long long *d_step = nullptr;

@@ -124,10 +124,6 @@ struct FillArgs {
   Layout L;
   void *f;               // state being filled (in place)
   const void *f2;        // the other buffer: the ghosts of the step before
-  const uint32_t *mask;
-  int nxw;
-  int wall_y, wall_z;
-  const void *f_in;      // inlet equilibrium, Q stored elements (channel profile)
 };
 
 struct LinkArgs {
@@ -174,7 +170,6 @@ constexpr int SWEEP_BX = 32, SWEEP_BY = 4;
 inline int sweep_rows(const Layout &L) {
   return (SWEEP_BY - 1) * L.rs + SWEEP_BX < (1LL << 32) ? SWEEP_BY : 1;
 }
-cudaError_t launch_fill_channel(int Q, int store, const FillArgs &a, cudaStream_t s);
 // The face passes op[0..nops) of a step and, with la.blocks > 0, its link fill, as one
 // launch (both only where neither reads what the other writes); several for faces
 // beyond FACE_THREADS.
@@ -194,7 +189,6 @@ cudaError_t launch_reduce_mass(int Q, int store, const ReduceArgs &a, int blocks
 // Rows [r0, r0 + n) of the dense [i][z][y][x] state to (or, put, from) `dense`.
 cudaError_t launch_dense_rows(int Q, int store, const Layout &L, void *f, double *dense,
                               long long r0, long long n, bool put, cudaStream_t s);
-cudaError_t launch_fill_value(int Q, int store, const Layout &L, void *f, cudaStream_t s);
 
 // Fill omega, omega_f and the relaxation constants rk/rkf and fx of a sweep for
 // lattice Q and arithmetic `compute` (ComputeKind; any storage: the codecs hand the
