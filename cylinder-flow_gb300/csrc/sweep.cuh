@@ -617,7 +617,7 @@ __device__ __forceinline__ void channel_listed_cell(const SweepArgs &a, int x, i
     rho3 = A(0); ux = A(0); uy = A(0); uz = A(0);
   }
   const long long cell = ((long long)z * ny + y) * nx + x;
-  finish_cell<L, SF, A, E, true>(f, rho3, ux, uy, uz, cell, valid, static_cast<E *>(a.fb), c, S, a);
+  finish_cell<L, SF, A, E>(f, rho3, ux, uy, uz, cell, valid, static_cast<E *>(a.fb), c, S, a);
 }
 
 // Interior channel sweep with two cells per thread and packed FP32x2
@@ -751,8 +751,8 @@ __device__ __forceinline__ void channel2_cells(const SweepArgs &a, int x0, int y
   }
   const long long cell0 = ((long long)z * ny + y) * nx + x0;
   // Fields out where asked for.  (No step asks: they are formed on request.  Without
-  // these lines the FP16 kernel's registers come out another way, 206.6 against 202.9
-  // us per step at 512x128x128, and a 64-channel batch takes 18.5 against 17.8 ms.)
+  // these lines the FP16 kernel's registers come out another way, 207.9 against 198.7
+  // us per step at 512x128x128, and a 64-channel batch takes 85.0 against 82.0.)
   if (a.mu) {
     if (st0) {
       a.mu[cell0] = T::to_double(T::x(ux));
@@ -1293,7 +1293,8 @@ cudaError_t launch_sweep_channel_t(const SweepArgs &a0, cudaStream_t s) {
     // 512x128x128 and 47.4 against 45.3 on 768x384x384 (5 per SM; 37.9 / 46.4
     // at 6), FP32 D2Q9 400x100 6.66 against 6.46 (5 per SM); FP32 D3Q27 the
     // same either way (31.0 / 32.2 at 6 per SM); the wide D2Q9 grids 1-2 %
-    // slower (8192x1024: FP16 129.5 against 130.8, FP32 91.4 against 93.3).
+    // slower (8192x1024: FP16 129.5 against 130.8, FP32 91.4 against 93.3); smaller FP16
+    // D2Q9 grids slower too (1021x241 4.23 against 3.16 us per step; FP32 3.21 / 3.23).
     if constexpr (Q == 27 && std::is_same<ST, float>::value)
       e = launch(sweep_channel2_kernel<Q, ST, float2, 6, false>);
     else if constexpr (Q == 27)
@@ -1301,7 +1302,7 @@ cudaError_t launch_sweep_channel_t(const SweepArgs &a0, cudaStream_t s) {
     else
       e = (long long)a.L.nx * a.L.ny >= (1LL << 20)
               ? launch(sweep_channel2_kernel<Q, ST, float2, 10, false>)
-              : launch(sweep_channel2_kernel<Q, ST, float2, 5, true>);
+              : launch(sweep_channel2_kernel<Q, ST, float2, 5, std::is_same<ST, float>::value>);
   } else if constexpr (Q == 9 && sizeof(A) == 4) {
     // FP64 storage: 94.3 / 89.4 / 87.1 us per step at 8 / 10 / 12 blocks per SM on
     // 4096x1024, 5.25 / 5.31 / 5.85 on 1021x241
