@@ -35,14 +35,19 @@ namespace cflbm {
 constexpr int FX_P = 55;             // q_i = g_i 2^(FX_P - E)
 constexpr int FX_EMAX = 1023 - 3;    // largest biased exponent covered
 constexpr int FX_EMIN = 1023 - 900;  // smaller ones are raised to it
-// Populations 0 .. fx_nint - 1 are converted to FP64 with integer operations, the
-// others by the FP64 pipe: with all 54 conversions of a D3Q27 cell on it that pipe
-// binds (27 clocks per cell and SM), with all 27 outgoing ones off it the integer
-// pipes do.  10 steps and the fields of the 512x128x128 cylinder, ms: 7.50 / 7.40 /
-// 7.33 / 7.36 / 7.39 for 18 / 20 / 22 / 25 / 27 (with a longer conversion 9.34 for
-// none, 8.39 for 18; FP64 operations: 22.78); D2Q9 1132x168, 400 steps: 3.31 / 3.24 /
-// 3.22 / 3.25 for 3 / 4 / 5 / 6 (FP64 operations: 4.01).
-template <class L> constexpr int fx_nint = L::D == 3 ? 22 : 5;
+// Populations that the FP64 pipe converts back; the others are converted with integer
+// operations: with all 54 conversions of a D3Q27 cell on that pipe it binds (27 clocks
+// per cell and SM), with all 27 outgoing ones off it the integer pipes do.  10 steps and
+// the fields of the 512x128x128 cylinder, ms: 7.50 / 7.40 / 7.33 / 7.36 / 7.39 with 9 / 7
+// / 5 / 2 / 0 there (with a longer conversion 9.34 for 27, 8.39 for 9; FP64 operations:
+// 22.78); D2Q9 1132x168, 400 steps: 3.31 / 3.24 / 3.22 / 3.25 with 6 / 5 / 4 / 3 (FP64
+// operations: 4.01).  The two round ties differently (to even; away from zero), so the
+// set holds with a direction its mirror images: populations that are equal stay equal,
+// and a flow uniform in z keeps w = 0.
+template <class L>
+__host__ __device__ constexpr bool fx_pipe(int i) {
+  return L::D == 3 ? L::ez(i) == 0 && wclass<L>(i) != 1 : wclass<L>(i) == 2;
+}
 
 // Shift of the weight of class c = |e|^2 (w = W 2^k), the scale of the velocity
 // sums (u = M 2^(E - FX_P - FX_U)) and of rho3 (FX_R).
@@ -266,7 +271,7 @@ __device__ __forceinline__ bool fixed_cell(const double *f, bool solid, bool inl
     constexpr int I = decltype(ic)::value;
     const long long x = mul_hi_b(limbs(q[I]), a.fx[FX_OMC], eq);
     double r;
-    if constexpr (I < fx_nint<L>) {
+    if constexpr (!fx_pipe<L>(I)) {
       r = fx_to_double(x, out20 + (1023 + Fx<L>::k(wclass<L>(I))) * (1 << 20));
     } else {
       const double d = __ll2double_rn(x);

@@ -144,3 +144,19 @@ def test_slow_relaxation_keeps_small_populations(cuda, lattice, dims, tau0):
     scale = w * np.abs(g / w).max(axis=0).astype(float)
     tol = 2.0 ** -53 * (2 * np.abs(g).astype(float) + 64 * omega * scale)
     assert (np.abs(got - ref).astype(float) <= tol)[..., 1:-1].all()
+
+
+@pytest.mark.parametrize("compute", ["fp64", "df64"])
+@pytest.mark.parametrize("wall_z", ["periodic", "freeslip"])
+def test_spanwise_uniform_flow_stays_so(cuda, wall_z, compute):
+    """Populations that mirror each other in z round alike, whichever pipe converts
+    them: a flow uniform in z keeps w = 0 and equal layers, to the bit."""
+    from cflbm import Solver
+    with Solver(lattice=27, nx=90, ny=34, nz=9, tau0=0.0192, u0=0.05, wall_z=wall_z, geom="cylinder", cx=24,
+                cy=15.3, diam=9, perturb_amp=0.0, compute=compute) as s:
+        s.step(120)
+        u, v, w, p = [np.asarray(m).reshape(9, 34, 90) for m in s.macros()]
+        f = s.get_f().reshape(27, 9, 34, 90)
+    assert np.abs(v).max() > 1e-3 and not w.any()
+    for m in (u, v, p, *f):
+        assert np.array_equal(m, np.broadcast_to(m[:1], m.shape))
