@@ -4,8 +4,8 @@
 // GB300 has two FP64 lanes per SM (measured 2.0 DFMA, 1.7 DADD and also 2.0
 // double <-> int64 conversions per clock and SM), against 64 integer additions
 // and about 18 32 x 32 -> 64-bit multiply-adds.  A D3Q27 update in FP64
-// arithmetic takes 133 instructions of that pipe; here it takes the 54
-// conversions (27 in, 27 out) and everything between runs on the integer pipes.
+// arithmetic takes 133 instructions of that pipe; here it takes 32 conversions (27
+// in, 5 out; fx_pipe) and everything else runs on the integer pipes.
 //
 // Format.  The weights of both lattices are one constant W times powers of two
 // (D3Q27: 1/27 x {8, 2, 1/2, 1/8}; D2Q9: 1/9 x {4, 1, 1/4}), so g_i = f_i 2^-k_i
@@ -20,8 +20,10 @@
 // sums of the q_i (headroom: 216 x 2^56 < 2^64 in units of the corner weight, rho3
 // at half that scale), the products are rounded 64 x 64 -> 64-bit high parts
 // with constants of 58 to 63 bits, and the relaxed populations come out in units
-// of 2^(E - 54), which one conversion rounds to 53 bits.  Every rounding is to
-// nearest, so no step adds a bias.
+// of 2^(E - 54), which one conversion rounds to 53 bits.  Roundings are to nearest,
+// ties up in the products, to even in the FP64 pipe's conversions and away from zero in
+// the integer one (at the largest populations two bits are dropped, so a quarter of
+// those values are ties); rho3's half is floored.
 //
 // Cells the format does not cover take the FP64 operations (bgk_relax_each):
 // |g_i| >= 1/4 (|u| well above 0.3), infinities and NaNs, and rates within 2^-20
