@@ -45,10 +45,13 @@ constexpr int FX_EMIN = 1023 - 900;  // smaller ones are raised to it
 // 22.78); D2Q9 1132x168, 400 steps: 3.31 / 3.24 / 3.22 / 3.25 with 6 / 5 / 4 / 3 (FP64
 // operations: 4.01).  The two round ties differently (to even; away from zero), so the
 // set holds with a direction its mirror images: populations that are equal stay equal,
-// and a flow uniform in z keeps w = 0.
+// and a flow uniform in z keeps w = 0.  Of such sets in D3Q27, rest and the yz / xz / xy
+// diagonals, rest and the x and y axes: 649 / 659 / 660 / 668 us per step at 512x128x128
+// (the last five by index, not closed: 666), 19.3 / 19.6 / 20.4 / 20.3 at 100x40x36
+// (19.9), REF3D 257x97x97 223.5 / 223.8 / 227.2 / 226.6 (226.3).
 template <class L>
 __host__ __device__ constexpr bool fx_pipe(int i) {
-  return L::D == 3 ? L::ez(i) == 0 && wclass<L>(i) != 1 : wclass<L>(i) == 2;
+  return L::D == 3 ? i == 0 || (L::ex(i) == 0 && wclass<L>(i) == 2) : wclass<L>(i) == 2;
 }
 
 // Shift of the weight of class c = |e|^2 (w = W 2^k), the scale of the velocity
