@@ -323,8 +323,8 @@ def run_gb300(args):
                      "bytes_per_cell": info.bytes_per_cell_step,
                      "sweep_us": round(sweep_s * 1e6, 2),
                      "note": "FP64 precision in block fixed point: the FP64 pipe (32 "
-                             "conversions per cell, 71 % active) and the integer pipe "
-                             "(63 %) bind together "
+                             "conversions per cell, 72 % active) and the integer pipe "
+                             "(64 %) bind together "
                              "(ncu, profiles/sweep_fp64_fixed_d3q27.md)"},
         "e2e": {"value": round(e2e_value, 2), "unit": "MLUPS", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "steps": e2e_steps, "forces_read_back": forces_ok,
